@@ -210,6 +210,19 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 //         FP16 operand mode).
 //   whn_l [WP][WP] FP32 W_l untransposed (j, k): the B operand of the
 //         backward GEMM d_in = d_a W_l.
+// Split section (FP32 on the tensor cores, level_split.cuh), phases in half
+// turns, omega / pi folded in (products taken in double):
+//   w0u   [4][WP]     rows W0[:,0..2], b0 times omega0 / pi, then the largest
+//                     magnitude of each row
+//   ws_l  FP16 parts of W_l omega_l / pi 2^k_l (level_split.cuh), hi and lo; K
+//         blocks of kSplitK, block kb and part p at ((2 kb + p) WP kSplitK + ((n/8) (kSplitK/8) + (k%kSplitK)/8) 64
+//         + (n%8) 8 + k%8) elements
+//   us_l  [WP]        omega_l / pi b_l
+//   eq_l  [WP]        2^p_n: hidden activations that can never exceed 2^-p_n are
+//         carried 2^p_n times larger, the next layer's column 2^-p_n smaller
+//   ub    [layers][4] bound of |phase| over the layer's rows, 2^-k_l, whether
+//         some p_n of the layer is not 0, unused
+constexpr int kSplitK = 32;
 struct PackLayout {
   int32_t L;    // nn.Linear layers
   int32_t WP;   // padded hidden width (64, 128 or 256)
@@ -222,6 +235,8 @@ struct PackLayout {
   int64_t hwh[MPL_MAX_LAYERS], hbxh[MPL_MAX_LAYERS];  // the same two tiles in FP16
   int64_t hwTh[MPL_MAX_LAYERS];                       // hwT in FP16
   int64_t whn[MPL_MAX_LAYERS];  // FP32 W_l as stored by nn.Linear, [j][k] (backward GEMM)
+  int64_t w0u, ub;
+  int64_t ws[MPL_MAX_LAYERS], us[MPL_MAX_LAYERS], eq[MPL_MAX_LAYERS];
   int64_t total;
 };
 

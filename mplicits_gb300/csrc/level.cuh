@@ -109,6 +109,7 @@ __device__ __forceinline__ void store_and_band(const LevelArgs& a, bool valid, i
 }
 
 int launch_level_fp32(const LevelArgs& a, cudaStream_t s);
+int launch_level_split(const LevelArgs& a, cudaStream_t s);
 int launch_level_bf16(const LevelArgs& a, cudaStream_t s);
 int launch_level_f16(const LevelArgs& a, cudaStream_t s);
 

@@ -1,5 +1,8 @@
 // Plain-form fused level evaluator: one SIREN level (i3d/model.py:88-129)
-// over a point tile, FP32 SIMT FMAs, accurate sinf.  One CTA per SM; a tile
+// over a point tile, FP32 SIMT FMAs, accurate sinf.  It serves the FP32
+// gradient and levels without a hidden GEMM; other FP32 levels run on the
+// tensor cores with split operands (level_split.cuh), ten times as fast and
+// with a smaller error.  One CTA per SM; a tile
 // is 128 rows x the padded width WP; activations stay in shared memory
 // between layers; hidden-layer weights are streamed from L2 as 32-row
 // K-chunks by the TMA engine into a double buffer.  Replaces the per-layer
@@ -336,6 +339,10 @@ int launch_fp32_mode(const LevelArgs& a, cudaStream_t s) {
 }  // namespace
 
 int launch_level_fp32(const LevelArgs& a, cudaStream_t s) {
+  if (!a.grad && a.lay.nh >= 1) {
+    const int st = launch_level_split(a, s);
+    if (st != MPL_ERR_UNSUPPORTED) return st;
+  }
   return a.grad ? launch_fp32_mode<true>(a, s) : launch_fp32_mode<false>(a, s);
 }
 

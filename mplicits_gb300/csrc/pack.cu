@@ -3,6 +3,7 @@
 // (renderer/cuda/gemms.cu:5-100, loaded by tools.cu:81-111).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <string.h>
 
 #include "common.cuh"
 
@@ -33,6 +34,7 @@ int make_layout(const MplNet* net, PackLayout* lay) {
   for (int l = 0; l < MPL_MAX_LAYERS; ++l) {
     lay->wht[l] = lay->bh[l] = lay->hb[l] = lay->hw[l] = lay->hwT[l] = lay->hbx[l] = -1;
     lay->hwh[l] = lay->hbxh[l] = lay->whn[l] = lay->hwTh[l] = -1;
+    lay->ws[l] = lay->us[l] = lay->eq[l] = -1;
   }
   for (int l = 1; l <= L - 2; ++l) {
     lay->wht[l] = take((int64_t)WP * WP * 4);
@@ -51,6 +53,13 @@ int make_layout(const MplNet* net, PackLayout* lay) {
     lay->whn[l] = take((int64_t)WP * WP * 4);
     lay->hwTh[l] = take((int64_t)WP * WP * 2);
   }
+  lay->w0u = take((4 * WP + 4) * 4);
+  lay->ub = take(MPL_MAX_LAYERS * 16);
+  for (int l = 1; l <= L - 2; ++l) {
+    lay->ws[l] = take((int64_t)WP * WP * 4);
+    lay->us[l] = take((int64_t)WP * 4);
+    lay->eq[l] = take((int64_t)WP * 4);
+  }
   lay->total = o;
   return MPL_OK;
 }
@@ -61,69 +70,164 @@ __device__ __forceinline__ int64_t umma_tile_offset(int n, int k, int WP) {
   return (int64_t)c * WP * 64 + ((int64_t)(n >> 3) * 8 + (kk >> 3)) * 64 + (n & 7) * 8 + (k & 7);
 }
 
-__global__ void pack_layer0(const float* __restrict__ W, const float* __restrict__ b, int out,
-                            int WP, float omega, float* w0t, float* b0, float* w0f) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= WP) return;
-  const bool v = j < out;
-  for (int c = 0; c < 3; ++c) {
-    float w = v ? W[j * 3 + c] : 0.f;
-    w0t[c * WP + j] = w;
-    w0f[c * WP + j] = omega * w;
-  }
-  float bb = v ? b[j] : 0.f;
-  b0[j] = bb;
-  w0f[3 * WP + j] = omega * bb;
+struct PackHidden {
+  const float *W, *b;
+  int out, in;
+  float omega;
+  double turns;  // omega / pi
+  float *wt, *bh, *hb, *whn, *us, *ub, *eq;
+  const float* eq_in;  // of the layer before; null for the first hidden one
+  __nv_bfloat16 *hw, *hwT, *hbx;
+  __half *hwh, *hwTh, *hbxh, *ws;
+};
+struct PackArgs {
+  const float *W0, *b0, *Wl, *bl;  // first and output layer
+  int out0, inl, WP;
+  float omega0;
+  double turns0;
+  float *w0t, *b0p, *w0f, *w0u, *wout, *bout;
+  PackHidden hid[MPL_MAX_LAYERS];
+};
+
+// maximum of non-negative v over the block (NaN ignored), to every thread
+__device__ __forceinline__ float block_max(float v) {
+  __shared__ float s[8];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = s[0];
+  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmaxf(v, s[w]);
+  return v;
 }
 
-__global__ void pack_hidden(const float* __restrict__ W, const float* __restrict__ b, int out,
-                            int in, int WP, float omega, float* wt, float* bh, float* hb,
-                            __nv_bfloat16* hw, __nv_bfloat16* hwT, __half* hwh, float* whn,
-                            __half* hwTh) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (int64_t)WP * WP) return;
-  const int n = (int)(e / WP), k = (int)(e % WP);  // n: output row, k: input col
-  const float w = (n < out && k < in) ? W[(int64_t)n * in + k] : 0.f;
-  wt[(int64_t)k * WP + n] = w;
-  whn[(int64_t)n * WP + k] = w;
-  hw[umma_tile_offset(n, k, WP)] = __float2bfloat16_rn(omega * w);
-  hwT[umma_tile_offset(k, n, WP)] = __float2bfloat16_rn(omega * w);
-  hwh[umma_tile_offset(n, k, WP)] = __float2half_rn(omega * w);
-  hwTh[umma_tile_offset(k, n, WP)] = __float2half_rn(omega * w);
+// e of the smallest 2^e that a magnitude does not exceed (up to rounding); 0 for
+// 0, an infinity or a NaN; within the range whose powers are normal floats
+__device__ __forceinline__ int magnitude_exponent(float m) {
+  int e = 0;
+  if (isfinite(m) && m > 0.f) frexpf(m, &e);
+  return e < -110 ? -110 : e;
+}
+
+// Row bounds of a hidden layer (blockIdx.y; one block of WP threads per row):
+// |phase| <= sum |w'| + |b'|, since activations are at most 1, and the power of
+// two that brings a small activation, at most pi times that, up to 1.
+__global__ void pack_rows(const PackArgs a) {
+  const PackHidden& h = a.hid[blockIdx.y];
+  const int n = blockIdx.x, k = threadIdx.x;
+  float sum = 0.f;
+  if (n < h.out && k < h.in) sum = fabsf((float)(h.turns * (double)h.W[(int64_t)n * h.in + k]));
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  __shared__ float part[8];
+  if ((k & 31) == 0) part[k >> 5] = sum;
+  __syncthreads();
   if (k == 0) {
-    const float bb = n < out ? b[n] : 0.f;
-    bh[n] = bb;
-    hb[n] = omega * bb;
+    const float bu = n < h.out ? (float)(h.turns * (double)h.b[n]) : 0.f;
+    float t = fabsf(bu);
+    for (int i = 0; i < a.WP / 32; ++i) t += part[i];
+    h.us[n] = bu;
+    // non-negative floats order as their bits, infinity and NaN last
+    atomicMax(reinterpret_cast<unsigned int*>(h.ub), __float_as_uint(fabsf(t)));
+    int p = -magnitude_exponent(t * 3.2f);
+    p = p < 0 ? 0 : (p > 60 ? 60 : p);
+    h.eq[n] = ldexpf(1.f, p);
+    if (p) h.ub[2] = 1.f;
   }
 }
 
-// bias tile of the MMA (see PackLayout::hbx): row n, K columns 0 and 1
-__global__ void pack_bias_tile(const float* __restrict__ b, int out, int WP, float omega,
-                               __nv_bfloat16* hbx, __half* hbxh) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= WP) return;
-  const float v = n < out ? omega * b[n] : 0.f;
-  const int base = ((n >> 3) * 2) * 64 + (n & 7) * 8;  // elements; K group 0
-  for (int k = 0; k < 8; ++k) {
-    hbx[base + k] = hbx[base + 64 + k] = __float2bfloat16_rn(0.f);
-    hbxh[base + k] = hbxh[base + 64 + k] = __float2half_rn(0.f);
-  }
-  const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-  hbx[base + 0] = hi;
-  hbx[base + 1] = __float2bfloat16_rn(v - __bfloat162float(hi));
-  const __half hh = __float2half_rn(v);
-  hbxh[base + 0] = hh;
-  hbxh[base + 1] = __float2half_rn(v - __half2float(hh));
+// omega / pi W of one element, the column scaled as its activation is
+__device__ __forceinline__ double split_weight(const PackHidden& h, float w, int k) {
+  const double u = h.turns * (double)w;
+  return h.eq_in ? u / (double)h.eq_in[k] : u;
 }
 
-__global__ void pack_output(const float* __restrict__ W, const float* __restrict__ b, int in,
-                            int WP, float* wout, float* bout) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < WP) wout[j] = j < in ? W[j] : 0.f;
-  if (j == 0) {
-    bout[0] = b[0];
-    bout[1] = bout[2] = bout[3] = 0.f;
+// largest such magnitude of each hidden layer into its ub[1] (zeroed before)
+__global__ void pack_range(const PackArgs a) {
+  const PackHidden& h = a.hid[blockIdx.y];
+  float m = 0.f;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < h.out * h.in;
+       i += gridDim.x * blockDim.x)
+    m = fmaxf(m, fabsf((float)split_weight(h, h.W[i], i % h.in)));
+  m = block_max(m);
+  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(h.ub + 1), __float_as_uint(m));
+}
+
+// 2^-k_l in place of the layers' largest magnitudes, after pack_level
+__global__ void pack_scales(const PackArgs a, int nh) {
+  const int l = threadIdx.x;
+  if (l < nh) a.hid[l].ub[1] = ldexpf(1.f, magnitude_exponent(a.hid[l].ub[1]) - 15);
+}
+
+// One block of WP threads per row of a hidden layer (blockIdx.y - 1), and one
+// (blockIdx.y = 0, x = 0) for the first and output layers: the whole image in
+// one launch (a training step packs the level it has just updated).
+__global__ void pack_level(const PackArgs a) {
+  const int WP = a.WP, k = threadIdx.x;
+  if (blockIdx.y == 0) {
+    if (blockIdx.x != 0) return;
+    const bool v = k < a.out0;
+    float mag[4];
+    for (int c = 0; c < 4; ++c) {
+      const float w = !v ? 0.f : (c < 3 ? a.W0[k * 3 + c] : a.b0[k]);
+      const float u = (float)(a.turns0 * (double)w);
+      if (c < 3)
+        a.w0t[c * WP + k] = w;
+      else
+        a.b0p[k] = w;
+      a.w0f[c * WP + k] = a.omega0 * w;
+      a.w0u[c * WP + k] = u;
+      // a NaN weight makes the bound infinite: such phases need no fast path
+      mag[c] = u == u ? fabsf(u) : INFINITY;
+    }
+    for (int c = 0; c < 4; ++c) {
+      const float mx = block_max(mag[c]);
+      if (k == 0) a.w0u[4 * WP + c] = mx;
+    }
+    a.wout[k] = k < a.inl ? a.Wl[k] : 0.f;
+    if (k < 4) a.bout[k] = k == 0 ? a.bl[0] : 0.f;
+    return;
   }
+  const PackHidden& h = a.hid[blockIdx.y - 1];
+  const int n = blockIdx.x;  // output row; k: input column
+  const float w = (n < h.out && k < h.in) ? h.W[(int64_t)n * h.in + k] : 0.f;
+  h.wt[(int64_t)k * WP + n] = w;
+  h.whn[(int64_t)n * WP + k] = w;
+  h.hw[umma_tile_offset(n, k, WP)] = __float2bfloat16_rn(h.omega * w);
+  h.hwT[umma_tile_offset(k, n, WP)] = __float2bfloat16_rn(h.omega * w);
+  h.hwh[umma_tile_offset(n, k, WP)] = __float2half_rn(h.omega * w);
+  h.hwTh[umma_tile_offset(k, n, WP)] = __float2half_rn(h.omega * w);
+  // bias tile of the MMA (PackLayout::hbx): row n, K columns 0 and 1 of 16
+  const float bb = n < h.out ? h.b[n] : 0.f;
+  const float v = h.omega * bb;
+  if (k < 16) {
+    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+    const __half hh = __float2half_rn(v);
+    const int at = ((n >> 3) * 2 + (k >> 3)) * 64 + (n & 7) * 8 + (k & 7);
+    h.hbx[at] = k == 0 ? hi
+                       : (k == 1 ? __float2bfloat16_rn(v - __bfloat162float(hi))
+                                 : __float2bfloat16_rn(0.f));
+    h.hbxh[at] = k == 0 ? hh : (k == 1 ? __float2half_rn(v - __half2float(hh))
+                                       : __float2half_rn(0.f));
+  }
+  if (k == 0) {
+    h.bh[n] = bb;
+    h.hb[n] = v;
+  }
+  // split parts: 2^k puts the layer's largest magnitude into [2^14, 2^15]; the
+  // row's hi parts are multiples of 2^(e - 11), e its own largest exponent
+  const double wu = split_weight(h, w, k);
+  const float mx = block_max(fabsf((float)wu));
+  const int k2 = 15 - magnitude_exponent(h.ub[1]);
+  const double wn = ldexp(wu, k2);
+  const double unit = ldexp(1.0, magnitude_exponent(mx) + k2 - 11);
+  const double hi = rint(wn / unit) * unit;
+  const int kk = k % kSplitK;
+  __half* dst = h.ws + (int64_t)(k / kSplitK) * 2 * WP * kSplitK +
+                ((n >> 3) * (kSplitK / 8) + (kk >> 3)) * 64 + (n & 7) * 8 + (kk & 7);
+  dst[0] = __double2half(hi);
+  dst[(int64_t)WP * kSplitK] = __double2half(wn - hi);
 }
 
 }  // namespace mpl
@@ -150,31 +254,63 @@ extern "C" int mpl_net_pack(const MplNet* net, const float* const* weights,
     if (!weights[l] || !biases[l]) return MPL_ERR_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   char* base = (char*)packed;
-  MPL_CUDA_TRY(cudaMemsetAsync(packed, 0, lay.total, s));
   const int WP = lay.WP;
-  pack_layer0<<<(WP + 127) / 128, 128, 0, s>>>(weights[0], biases[0], net->dims[1], WP,
-                                                net->omega[0], (float*)(base + lay.w0t),
-                                                (float*)(base + lay.b0), (float*)(base + lay.w0f));
-  MPL_LAUNCH_CHECK();
-  for (int l = 1; l <= lay.L - 2; ++l) {
-    const int64_t n = (int64_t)WP * WP;
-    pack_hidden<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-        weights[l], biases[l], net->dims[l + 1], net->dims[l], WP, net->omega[l],
-        (float*)(base + lay.wht[l]), (float*)(base + lay.bh[l]), (float*)(base + lay.hb[l]),
-        (__nv_bfloat16*)(base + lay.hw[l]), (__nv_bfloat16*)(base + lay.hwT[l]),
-        (__half*)(base + lay.hwh[l]), (float*)(base + lay.whn[l]),
-        (__half*)(base + lay.hwTh[l]));
+  PackArgs a;
+  memset(&a, 0, sizeof(a));
+  a.WP = WP;
+  a.W0 = weights[0];
+  a.b0 = biases[0];
+  a.Wl = weights[lay.L - 1];
+  a.bl = biases[lay.L - 1];
+  a.out0 = net->dims[1];
+  a.inl = net->dims[lay.L - 1];
+  constexpr double kInvPi = 0.31830988618379067154;
+  a.omega0 = net->omega[0];
+  a.turns0 = (double)net->omega[0] * kInvPi;
+  auto f32 = [&](int64_t off) { return (float*)(base + off); };
+  a.w0t = f32(lay.w0t);
+  a.b0p = f32(lay.b0);
+  a.w0f = f32(lay.w0f);
+  a.w0u = f32(lay.w0u);
+  a.wout = f32(lay.wout);
+  a.bout = f32(lay.bout);
+  for (int l = 1; l <= lay.nh; ++l) {
+    PackHidden& h = a.hid[l - 1];
+    h.W = weights[l];
+    h.b = biases[l];
+    h.out = net->dims[l + 1];
+    h.in = net->dims[l];
+    h.omega = net->omega[l];
+    h.turns = (double)net->omega[l] * kInvPi;
+    h.wt = f32(lay.wht[l]);
+    h.bh = f32(lay.bh[l]);
+    h.hb = f32(lay.hb[l]);
+    h.whn = f32(lay.whn[l]);
+    h.us = f32(lay.us[l]);
+    h.ub = f32(lay.ub) + 4 * l;
+    h.eq = f32(lay.eq[l]);
+    h.eq_in = l > 1 ? f32(lay.eq[l - 1]) : nullptr;
+    h.hw = (__nv_bfloat16*)(base + lay.hw[l]);
+    h.hwT = (__nv_bfloat16*)(base + lay.hwT[l]);
+    h.hbx = (__nv_bfloat16*)(base + lay.hbx[l]);
+    h.hwh = (__half*)(base + lay.hwh[l]);
+    h.hwTh = (__half*)(base + lay.hwTh[l]);
+    h.hbxh = (__half*)(base + lay.hbxh[l]);
+    h.ws = (__half*)(base + lay.ws[l]);
+  }
+  MPL_CUDA_TRY(cudaMemsetAsync(base + lay.ub, 0, MPL_MAX_LAYERS * 16, s));  // maxima
+  const dim3 grid(lay.nh > 0 ? WP : 1, 1 + lay.nh);
+  if (lay.nh > 0) {
+    pack_rows<<<dim3(WP, lay.nh), WP, 0, s>>>(a);
     MPL_LAUNCH_CHECK();
-    pack_bias_tile<<<(WP + 127) / 128, 128, 0, s>>>(biases[l], net->dims[l + 1], WP,
-                                                    net->omega[l],
-                                                    (__nv_bfloat16*)(base + lay.hbx[l]),
-                                                    (__half*)(base + lay.hbxh[l]));
+    pack_range<<<dim3(16, lay.nh), 256, 0, s>>>(a);
     MPL_LAUNCH_CHECK();
   }
-  pack_output<<<(WP + 127) / 128, 128, 0, s>>>(weights[lay.L - 1], biases[lay.L - 1],
-                                                net->dims[lay.L - 1], WP,
-                                                (float*)(base + lay.wout),
-                                                (float*)(base + lay.bout));
+  pack_level<<<grid, WP, 0, s>>>(a);
   MPL_LAUNCH_CHECK();
+  if (lay.nh > 0) {
+    pack_scales<<<1, 32, 0, s>>>(a, lay.nh);
+    MPL_LAUNCH_CHECK();
+  }
   return MPL_OK;
 }

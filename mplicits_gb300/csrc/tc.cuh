@@ -88,6 +88,43 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
       : "memory");
 }
 
+// The same for a warp that issues as one: every lane runs the code around it
+// (so descriptors, counters and waits stay warp-uniform and live in uniform
+// registers, which the instruction takes its operands from) and only the lane
+// with `lead` set issues.  Issued from inside an `if (lane == 0)` branch, each
+// descriptor is moved there one by one: about 200 cycles a K = 16 step of a
+// 128 x 256 tile, where the tensor cores need 128.
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(p));
+  return p;
+}
+
+__device__ __forceinline__ void mma_lead(uint32_t lead, uint32_t d_tmem, uint64_t adesc,
+                                         uint64_t bdesc, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(lead)
+      : "memory");
+}
+
+__device__ __forceinline__ void commit_lead(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          (uint32_t)__cvta_generic_to_shared(bar)),
+      "r"(lead)
+      : "memory");
+}
+
 // 32 lanes x 32 consecutive 32-bit columns: lane i of the warp receives
 // row (lane base + i), columns col..col+31.
 __device__ __forceinline__ void ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
