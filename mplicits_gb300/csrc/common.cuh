@@ -220,8 +220,8 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 //   us_l  [WP]        omega_l / pi b_l
 //   eq_l  [WP]        2^p_n: hidden activations that can never exceed 2^-p_n are
 //         carried 2^p_n times larger, the next layer's column 2^-p_n smaller
-//   ub    [layers][4] bound of |phase| over the layer's rows, 2^-k_l, whether
-//         some p_n of the layer is not 0, unused
+//   ub    [layers][4] bound of |phase| over the layer's rows, largest |omega / pi
+//         W 2^-p|, whether some p_n of the layer is not 0, 2^-k_l
 constexpr int kSplitK = 32;
 struct PackLayout {
   int32_t L;    // nn.Linear layers

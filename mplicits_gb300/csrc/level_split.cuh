@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1) level_split_kernel(const LevelArg
     auto read_phases = [&](int l) {
       const float* bias = us + (l - 1) * WP;
       const float* lay = reinterpret_cast<const float*>(pk + a.lay.ub) + 4 * l;
-      const uint64_t scale = both(lay[1]);
+      const uint64_t scale = both(lay[3]);
       const bool far = !(lay[0] <= kPhaseLimit);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {

@@ -137,27 +137,25 @@ __global__ void pack_rows(const PackArgs a) {
   }
 }
 
+// 2^e, |e| <= 1022
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
 // omega / pi W of one element, the column scaled as its activation is
 __device__ __forceinline__ double split_weight(const PackHidden& h, float w, int k) {
   const double u = h.turns * (double)w;
-  return h.eq_in ? u / (double)h.eq_in[k] : u;
+  return h.eq_in ? u * (double)__frcp_rn(h.eq_in[k]) : u;  // a power of two: exact
 }
 
-// largest such magnitude of each hidden layer into its ub[1] (zeroed before)
+// largest such magnitude of each hidden layer into its ub[1] (zeroed before);
+// one block of WP threads per row
 __global__ void pack_range(const PackArgs a) {
   const PackHidden& h = a.hid[blockIdx.y];
+  const int n = blockIdx.x, k = threadIdx.x;
   float m = 0.f;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < h.out * h.in;
-       i += gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf((float)split_weight(h, h.W[i], i % h.in)));
+  if (n < h.out && k < h.in)
+    m = fabsf((float)split_weight(h, h.W[(int64_t)n * h.in + k], k));
   m = block_max(m);
-  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(h.ub + 1), __float_as_uint(m));
-}
-
-// 2^-k_l in place of the layers' largest magnitudes, after pack_level
-__global__ void pack_scales(const PackArgs a, int nh) {
-  const int l = threadIdx.x;
-  if (l < nh) a.hid[l].ub[1] = ldexpf(1.f, magnitude_exponent(a.hid[l].ub[1]) - 15);
+  if (k == 0) atomicMax(reinterpret_cast<unsigned int*>(h.ub + 1), __float_as_uint(m));
 }
 
 // One block of WP threads per row of a hidden layer (blockIdx.y - 1), and one
@@ -220,14 +218,15 @@ __global__ void pack_level(const PackArgs a) {
   const double wu = split_weight(h, w, k);
   const float mx = block_max(fabsf((float)wu));
   const int k2 = 15 - magnitude_exponent(h.ub[1]);
-  const double wn = ldexp(wu, k2);
-  const double unit = ldexp(1.0, magnitude_exponent(mx) + k2 - 11);
-  const double hi = rint(wn / unit) * unit;
+  if (n == 0 && k == 0) h.ub[3] = (float)pow2(-k2);
+  const double wn = wu * pow2(k2);
+  const int eu = magnitude_exponent(mx) + k2 - 11;
+  const double hi = rint(wn * pow2(-eu)) * pow2(eu);
   const int kk = k % kSplitK;
   __half* dst = h.ws + (int64_t)(k / kSplitK) * 2 * WP * kSplitK +
                 ((n >> 3) * (kSplitK / 8) + (kk >> 3)) * 64 + (n & 7) * 8 + (kk & 7);
-  dst[0] = __double2half(hi);
-  dst[(int64_t)WP * kSplitK] = __double2half(wn - hi);
+  dst[0] = __float2half_rn((float)hi);
+  dst[(int64_t)WP * kSplitK] = __float2half_rn((float)(wn - hi));
 }
 
 }  // namespace mpl
@@ -298,19 +297,15 @@ extern "C" int mpl_net_pack(const MplNet* net, const float* const* weights,
     h.hbxh = (__half*)(base + lay.hbxh[l]);
     h.ws = (__half*)(base + lay.ws[l]);
   }
-  MPL_CUDA_TRY(cudaMemsetAsync(base + lay.ub, 0, MPL_MAX_LAYERS * 16, s));  // maxima
+  MPL_CUDA_TRY(cudaMemsetAsync(base + lay.ub, 0, MPL_MAX_LAYERS * 16, s));  // maxima, flags
   const dim3 grid(lay.nh > 0 ? WP : 1, 1 + lay.nh);
   if (lay.nh > 0) {
     pack_rows<<<dim3(WP, lay.nh), WP, 0, s>>>(a);
     MPL_LAUNCH_CHECK();
-    pack_range<<<dim3(16, lay.nh), 256, 0, s>>>(a);
+    pack_range<<<dim3(WP, lay.nh), WP, 0, s>>>(a);
     MPL_LAUNCH_CHECK();
   }
   pack_level<<<grid, WP, 0, s>>>(a);
   MPL_LAUNCH_CHECK();
-  if (lay.nh > 0) {
-    pack_scales<<<1, 32, 0, s>>>(a, lay.nh);
-    MPL_LAUNCH_CHECK();
-  }
   return MPL_OK;
 }
