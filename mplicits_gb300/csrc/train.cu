@@ -43,6 +43,11 @@ struct TrainArgs {
   int* status;
 };
 
+struct WgradOut {
+  float* dW[MPL_MAX_LAYERS];
+  float* db[MPL_MAX_LAYERS];
+};
+
 // d_out of the last hidden layer from the seeds, then down the layers.
 template <int WP>
 __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const TrainArgs a) {
@@ -196,70 +201,123 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
   }
 }
 
-// in_l of a hidden layer l >= 1 for row ch of a point, feature k, from the
-// pre-activations of layer l-1: value sin(w a_v), tangent w cos(w a_v) a_t.
-__device__ __forceinline__ float layer_input(const float* pre_prev_point, int WP, int ch, int k,
-                                             float om) {
-  const float zv = __fmul_rn(om, pre_prev_point[k]);
-  if (ch == 0) return sinf(zv);
-  return __fmul_rn(__fmul_rn(om, cosf(zv)), pre_prev_point[ch * WP + k]);
-}
-
 // dW_l[j][k] += sum over rows of da_l[row][j] * in_l[row][k] (l >= 1), and
-// db_l[j] += sum over points of da_l[value row][j].  CTA tile 64 x 64,
-// split over points by blockIdx.z, partial sums added atomically.
-__global__ void __launch_bounds__(256) train_wgrad_hidden_kernel(const TrainArgs a, int l, int WP,
-                                                                 float* dW, float* db) {
-  __shared__ float sA[32][65];  // d_a rows x j
-  __shared__ float sB[32][65];  // in rows x k
-  const int j0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
+// db_l[j] += sum over points of da_l[value row][j], for every hidden layer in
+// one launch: blockIdx.y is the layer and the tile, blockIdx.x the points.
+// in_l comes from the pre-activations of layer l-1 (value sin(w a_v), tangent
+// w cos(w a_v) a_t), one sincosf per point and feature.  A CTA holds a T x T
+// tile of dW in registers (T/16 squared per thread) and walks its points four
+// at a time (16 rows), the next ones on their way while the products run;
+// partial sums go out as 16-byte atomic adds.
+// Bound: the FP32 FMA pipe.  The split over points fills two CTAs per SM
+// (train_wgrad_blocks): with a fixed 4096 points a CTA, 64 x 64 tiles and a
+// sine per row, 15,000 points of a 256-wide level took 3.25 ms a layer on 64
+// CTAs; now 0.24 ms on 304 (a whole FP32 training step 8.6 -> 2.5 ms).
+template <int T>
+__global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainArgs a, int WP,
+                                                                    WgradOut out) {
+  constexpr int E = T / 16;            // values of each axis per thread
+  constexpr int kGroup = 4;            // points per step
+  constexpr int kItems = kGroup * T / 256;  // (point, feature) pairs per thread
+  __shared__ __align__(16) float sA[2][4 * kGroup][T];  // d_a rows x j
+  __shared__ __align__(16) float sB[2][4 * kGroup][T];  // in rows x k
+  const int tiles = WP / T;
+  const int l = 1 + blockIdx.y / (tiles * tiles);
+  const int tile = blockIdx.y % (tiles * tiles);
+  const int j0 = (tile / tiles) * T, k0 = (tile % tiles) * T;
   const int tid = threadIdx.x, tj = tid >> 4, tk = tid & 15;
-  const int64_t per = (a.n + gridDim.z - 1) / gridDim.z;
-  const int64_t q_begin = blockIdx.z * per;
+  const int64_t per = ((a.n + gridDim.x - 1) / gridDim.x + kGroup - 1) / kGroup * kGroup;
+  const int64_t q_begin = blockIdx.x * per;
   const int64_t q_end = q_begin + per < a.n ? q_begin + per : a.n;
-  const float omp = a.omega[l - 1];
-  float acc[4][4] = {};
+  if (q_begin >= q_end) return;
+  const float om = a.omega[l - 1];
+  const float* da = a.da + (int64_t)l * a.n * 4 * WP + j0;
+  const float* pre = a.pre + (int64_t)(l - 1) * a.n * 4 * WP + k0;
+  float acc[E][E] = {};
   float bacc = 0.f;
-  for (int64_t q0 = q_begin; q0 < q_end; q0 += 8) {
-    // 8 points = 32 rows
-    for (int e = tid; e < 32 * 64; e += 256) {
-      const int r = e >> 6, c = e & 63;
-      const int64_t q = q0 + (r >> 2);
-      float va = 0.f, vb = 0.f;
-      if (q < q_end) {
-        va = a.da[(((int64_t)l * a.n + q) * 4 + (r & 3)) * WP + j0 + c];
-        vb = layer_input(a.pre + (((int64_t)(l - 1) * a.n + q) * 4) * WP, WP, r & 3, k0 + c, omp);
+  float ra[kItems][4], rb[kItems][4];
+  auto load = [&](int64_t q0) {
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const int e = tid + 256 * i, c = e % T;
+      const int64_t q = q0 + e / T;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const bool in = q < q_end;
+        ra[i][r] = in ? da[(q * 4 + r) * WP + c] : 0.f;
+        rb[i][r] = in ? pre[(q * 4 + r) * WP + c] : 0.f;
       }
-      sA[r][c] = va;
-      sB[r][c] = vb;
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int r = 0; r < 32; ++r) {
-      float av[4], bv[4];
+  };
+  auto stage = [&](int buf) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        av[u] = sA[r][tj * 4 + u];
-        bv[u] = sB[r][tk * 4 + u];
+    for (int i = 0; i < kItems; ++i) {
+      const int e = tid + 256 * i, c = e % T, row = 4 * (e / T);
+      float s, co;
+      sincosf(__fmul_rn(om, rb[i][0]), &s, &co);
+      co = __fmul_rn(om, co);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        sA[buf][row + r][c] = ra[i][r];
+        sB[buf][row + r][c] = r == 0 ? s : __fmul_rn(co, rb[i][r]);
+      }
+    }
+  };
+  load(q_begin);
+  stage(0);
+  __syncthreads();
+  int buf = 0;
+  for (int64_t q0 = q_begin; q0 < q_end; q0 += kGroup, buf ^= 1) {
+    const bool more = q0 + kGroup < q_end;
+    if (more) load(q0 + kGroup);
+#pragma unroll 4
+    for (int r = 0; r < 4 * kGroup; ++r) {
+      float av[E], bv[E];
+#pragma unroll
+      for (int u = 0; u < E; u += 4) {
+        // features 4 t .. + 3 of each half of the tile: 16-byte reads without
+        // bank conflicts
+        const float4 x = *reinterpret_cast<const float4*>(&sA[buf][r][u * 16 + tj * 4]);
+        const float4 y = *reinterpret_cast<const float4*>(&sB[buf][r][u * 16 + tk * 4]);
+        av[u] = x.x, av[u + 1] = x.y, av[u + 2] = x.z, av[u + 3] = x.w;
+        bv[u] = y.x, bv[u + 1] = y.y, bv[u + 2] = y.z, bv[u + 3] = y.w;
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < E; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = __fmaf_rn(av[u], bv[v], acc[u][v]);
+        for (int v = 0; v < E; ++v) acc[u][v] = __fmaf_rn(av[u], bv[v], acc[u][v]);
     }
-    if (blockIdx.y == 0 && tid < 64) {
-      for (int r = 0; r < 32; r += 4) bacc += sA[r][tid];
+    if (k0 == 0 && tid < T) {
+#pragma unroll
+      for (int r = 0; r < 4 * kGroup; r += 4) bacc += sA[buf][r][tid];
     }
+    if (more) stage(buf ^ 1);
     __syncthreads();
   }
+  float* dW = out.dW[l];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < E; ++u) {
+    const int j = j0 + (u / 4) * 64 + tj * 4 + (u & 3);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int j = j0 + tj * 4 + u, k = k0 + tk * 4 + v;
-      atomicAdd(&dW[(int64_t)j * WP + k], acc[u][v]);
-    }
-  if (blockIdx.y == 0 && tid < 64) atomicAdd(&db[j0 + tid], bacc);
+    for (int v = 0; v < E; v += 4)
+      atomicAdd(reinterpret_cast<float4*>(dW + (int64_t)j * WP + k0 + v * 16 + tk * 4),
+                make_float4(acc[u][v], acc[u][v + 1], acc[u][v + 2], acc[u][v + 3]));
+  }
+  if (k0 == 0 && tid < T) atomicAdd(&out.db[l][j0 + tid], bacc);
+}
+
+// Blocks that share the points of one tile: two per SM over all tiles, of 64
+// points at least (less would be mostly the atomic adds of the tile).
+template <int T>
+int launch_wgrad(const TrainArgs& t, int WP, const WgradOut& out, cudaStream_t s) {
+  const int per_layer = (WP / T) * (WP / T), all = per_layer * t.lay.nh;
+  int64_t splits = (2 * (int64_t)sm_count() + all - 1) / all;
+  const int64_t most = (t.n + 63) / 64;
+  splits = splits < most ? splits : most;
+  train_wgrad_hidden_kernel<T>
+      <<<dim3((unsigned)splits, (unsigned)all), 256, 0, s>>>(t, WP, out);
+  MPL_LAUNCH_CHECK();
+  return MPL_OK;
 }
 
 // Layer 0 (3 inputs): dW0[j][c] += sum_q da_v[j] x_qc + da_tc[j]; db0[j] += da_v[j].
@@ -529,11 +587,11 @@ extern "C" int mpl_train_backward(const MplNet* net, const void* packed, const f
     default: return MPL_ERR_UNSUPPORTED;
   }
   if (st != MPL_OK) return st;
-  const int splits = (int)((n + 4095) / 4096) < 64 ? (int)((n + 4095) / 4096) : 64;
-  for (int l = 1; l <= nh; ++l) {
-    dim3 grid(WP / 64, WP / 64, splits < 1 ? 1 : splits);
-    train_wgrad_hidden_kernel<<<grid, 256, 0, s>>>(t, l, WP, dW[l], db[l]);
-    MPL_LAUNCH_CHECK();
+  if (nh > 0) {
+    WgradOut out;
+    for (int l = 0; l < L; ++l) out.dW[l] = dW[l], out.db[l] = db[l];
+    st = WP == 64 ? launch_wgrad<64>(t, WP, out, s) : launch_wgrad<128>(t, WP, out, s);
+    if (st != MPL_OK) return st;
   }
   // about 64 points per block
   const int64_t eb = (n + 63) / 64 < 4096 ? (n + 63) / 64 : 4096;
