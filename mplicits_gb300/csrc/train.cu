@@ -19,7 +19,7 @@
 #include <math.h>
 #include <string.h>
 
-#include "level.cuh"
+#include "level_bf16.cuh"
 #include "train_loss.cuh"
 
 namespace mpl {
@@ -28,7 +28,6 @@ namespace {
 
 constexpr int kRows = 128;  // rows per tile = 32 points x 4
 constexpr int kPts = 32;
-constexpr int kThreads = 256;
 constexpr int kKC = 32;
 
 struct TrainArgs {
@@ -49,9 +48,14 @@ struct WgradOut {
 };
 
 // d_out of the last hidden layer from the seeds, then down the layers.
+// A thread holds 8 rows x 8 features (two groups of four, 4 TX apart), as in
+// the forward kernel; with 16 features a thread, half the warps, the tile's
+// latencies stood open (15,000 points of a 256-wide level 450 -> 429 us).
 template <int WP>
-__global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const TrainArgs a) {
-  constexpr int FPT = WP / 16;
+__global__ void __launch_bounds__(2 * WP, 1) train_backward_kernel(const TrainArgs a) {
+  constexpr int TX = WP / 8;
+  constexpr int kThreads = 16 * TX;
+  constexpr int FPT = 8;
   constexpr int NQ = FPT / 4;
   constexpr int CPL = WP / kKC;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -59,7 +63,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
   float* wbuf = act + WP * kRows;                // [2][KC][WP]
   float* wout = wbuf + 2 * kKC * WP;             // [WP]
   uint64_t* bar = reinterpret_cast<uint64_t*>(wout + WP);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int nh = a.lay.nh;
   const int64_t ntiles = (a.n + kPts - 1) / kPts;
   if ((int64_t)blockIdx.x >= ntiles) return;
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
       const int64_t q = t * kPts + (row >> 2);
       const float sd = q < a.n ? a.seed[q * 4 + (i & 3)] : 0.f;
 #pragma unroll
-      for (int f = 0; f < FPT; ++f) dout[i][f] = sd * wout[tx * 4 + (f & 3) + 64 * (f >> 2)];
+      for (int f = 0; f < FPT; ++f) dout[i][f] = sd * wout[tx * 4 + (f & 3) + 4 * TX * (f >> 2)];
     }
     for (int l = nh; l >= 0 && ok; --l) {
       const float om = a.omega[l];
@@ -114,7 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
         float* dar = a.da + (((int64_t)l * a.n + q) * 4) * WP;
 #pragma unroll
         for (int f4 = 0; f4 < FPT / 4; ++f4) {
-          const int j = tx * 4 + 64 * f4;
+          const int j = tx * 4 + 4 * TX * f4;
           float4 av[4] = {make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0),
                           make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0)};
           if (valid) {
@@ -159,11 +163,13 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
       }
       if (l == 0) break;
       __syncthreads();
-      // d_out of layer l-1 = d_a W_l (K = this layer's features)
+      // d_out of layer l-1 = d_a W_l (K = this layer's features), two features
+      // per FMA instruction as in the forward kernel
+      uint64_t dout2[8][FPT / 2];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int f = 0; f < FPT; ++f) dout[i][f] = 0.f;
+        for (int f = 0; f < FPT / 2; ++f) dout2[i][f] = 0ull;
       for (int c = 0; c < CPL; ++c, ++g) {
         if (tid == 0 && g + 1 < total) {
           issue(g + 1);
@@ -174,26 +180,33 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
           ok = false;
           break;
         }
-        const float4* w4 = reinterpret_cast<const float4*>(wbuf + (g & 1) * kKC * WP);
+        const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(wbuf + (g & 1) * kKC * WP);
         const int k0 = c * kKC;
 #pragma unroll 4
         for (int kk = 0; kk < kKC; ++kk) {
           const float4 a0 = act4[(k0 + kk) * (kRows / 4) + ty];
           const float4 a1 = act4[(k0 + kk) * (kRows / 4) + 16 + ty];
-          const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+          const uint64_t av[8] = {bf16::f2pack(a0.x, a0.x), bf16::f2pack(a0.y, a0.y),
+                                  bf16::f2pack(a0.z, a0.z), bf16::f2pack(a0.w, a0.w),
+                                  bf16::f2pack(a1.x, a1.x), bf16::f2pack(a1.y, a1.y),
+                                  bf16::f2pack(a1.z, a1.z), bf16::f2pack(a1.w, a1.w)};
 #pragma unroll
           for (int q4 = 0; q4 < NQ; ++q4) {
-            const float4 w = w4[kk * (WP / 4) + tx + 16 * q4];
-            const float wv[4] = {w.x, w.y, w.z, w.w};
+            const ulonglong2 w = w4[kk * (WP / 4) + tx + TX * q4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-              for (int r = 0; r < 4; ++r)
-                dout[i][q4 * 4 + r] = __fmaf_rn(av[i], wv[r], dout[i][q4 * 4 + r]);
+            for (int i = 0; i < 8; ++i) {
+              dout2[i][2 * q4] = bf16::ffma2(av[i], w.x, dout2[i][2 * q4]);
+              dout2[i][2 * q4 + 1] = bf16::ffma2(av[i], w.y, dout2[i][2 * q4 + 1]);
+            }
           }
         }
         __syncthreads();
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int f = 0; f < FPT / 2; ++f)
+          bf16::f2unpack(dout2[i][f], dout[i][2 * f], dout[i][2 * f + 1]);
     }
   }
   if (!ok && tid == 0) {
@@ -212,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_backward_kernel(const Train
 // Bound: the FP32 FMA pipe.  The split over points fills two CTAs per SM
 // (train_wgrad_blocks): with a fixed 4096 points a CTA, 64 x 64 tiles and a
 // sine per row, 15,000 points of a 256-wide level took 3.25 ms a layer on 64
-// CTAs; now 0.24 ms on 304 (a whole FP32 training step 8.6 -> 2.5 ms).
+// CTAs; now 0.16 ms on 304.
 template <int T>
 __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainArgs a, int WP,
                                                                     WgradOut out) {
@@ -233,7 +246,7 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
   const float om = a.omega[l - 1];
   const float* da = a.da + (int64_t)l * a.n * 4 * WP + j0;
   const float* pre = a.pre + (int64_t)(l - 1) * a.n * 4 * WP + k0;
-  float acc[E][E] = {};
+  uint64_t acc[E][E / 2] = {};  // two k per FMA instruction
   float bacc = 0.f;
   float ra[kItems][4], rb[kItems][4];
   auto load = [&](int64_t q0) {
@@ -272,20 +285,21 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
     if (more) load(q0 + kGroup);
 #pragma unroll 4
     for (int r = 0; r < 4 * kGroup; ++r) {
-      float av[E], bv[E];
+      uint64_t av[E], bv[E / 2];
 #pragma unroll
       for (int u = 0; u < E; u += 4) {
         // features 4 t .. + 3 of each half of the tile: 16-byte reads without
         // bank conflicts
         const float4 x = *reinterpret_cast<const float4*>(&sA[buf][r][u * 16 + tj * 4]);
-        const float4 y = *reinterpret_cast<const float4*>(&sB[buf][r][u * 16 + tk * 4]);
-        av[u] = x.x, av[u + 1] = x.y, av[u + 2] = x.z, av[u + 3] = x.w;
-        bv[u] = y.x, bv[u + 1] = y.y, bv[u + 2] = y.z, bv[u + 3] = y.w;
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(&sB[buf][r][u * 16 + tk * 4]);
+        av[u] = bf16::f2pack(x.x, x.x), av[u + 1] = bf16::f2pack(x.y, x.y);
+        av[u + 2] = bf16::f2pack(x.z, x.z), av[u + 3] = bf16::f2pack(x.w, x.w);
+        bv[u / 2] = y.x, bv[u / 2 + 1] = y.y;
       }
 #pragma unroll
       for (int u = 0; u < E; ++u)
 #pragma unroll
-        for (int v = 0; v < E; ++v) acc[u][v] = __fmaf_rn(av[u], bv[v], acc[u][v]);
+        for (int v = 0; v < E / 2; ++v) acc[u][v] = bf16::ffma2(av[u], bv[v], acc[u][v]);
     }
     if (k0 == 0 && tid < T) {
 #pragma unroll
@@ -299,9 +313,12 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
   for (int u = 0; u < E; ++u) {
     const int j = j0 + (u / 4) * 64 + tj * 4 + (u & 3);
 #pragma unroll
-    for (int v = 0; v < E; v += 4)
-      atomicAdd(reinterpret_cast<float4*>(dW + (int64_t)j * WP + k0 + v * 16 + tk * 4),
-                make_float4(acc[u][v], acc[u][v + 1], acc[u][v + 2], acc[u][v + 3]));
+    for (int v = 0; v < E; v += 4) {
+      float4 p;
+      bf16::f2unpack(acc[u][v / 2], p.x, p.y);
+      bf16::f2unpack(acc[u][v / 2 + 1], p.z, p.w);
+      atomicAdd(reinterpret_cast<float4*>(dW + (int64_t)j * WP + k0 + v * 16 + tk * 4), p);
+    }
   }
   if (k0 == 0 && tid < T) atomicAdd(&out.db[l][j0 + tid], bacc);
 }
@@ -498,7 +515,7 @@ int launch_backward_wp(const TrainArgs& t, cudaStream_t s) {
   int64_t grid = sm_count();
   const int64_t ntiles = (t.n + kPts - 1) / kPts;
   grid = ntiles < grid ? ntiles : grid;
-  train_backward_kernel<WP><<<(unsigned)grid, kThreads, smem, s>>>(t);
+  train_backward_kernel<WP><<<(unsigned)grid, 2 * WP, smem, s>>>(t);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
 }
