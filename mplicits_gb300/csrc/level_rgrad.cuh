@@ -15,11 +15,18 @@
 //             df/dx = (w0 W0)^T dz_0                    (FP32, z_0 recomputed)
 // The adjoints dz_l enter the backward GEMMs as 16-bit A operands against
 // the transposed weight tiles (omega folded in), as the activations enter
-// the forward ones.  One tile in flight per CTA; the GEMMs of a tile run in
-// sequence G_1 .. G_nh, B_nh .. B_1 into two TMEM accumulators (G_l and B_l
-// into accumulator (l - 1) & 1), so z_1 stays in accumulator 0 until B_2's
-// drain reads it (nh <= 2).  The next tile's first layer is written inside
-// the last drain.  Roles, waits and abort handling as in level_bf16.cuh.
+// the forward ones.  One tile is in flight per CTA, its GEMMs in sequence G_1 ..
+// G_nh, B_nh .. B_1 into two TMEM accumulators (G_l and B_l into the same one),
+// so z_1 stays where it is until B_2's drain reads it (nh <= 2).
+// Bound: the sine unit and the chain of GEMMs and drains.  A tile takes 1536
+// sines and cosines a row (12.3k cycles at 16 a cycle and SM) and 8.2k cycles of
+// MMA at width 256.  Two groups of epilogue warps split each drain: one takes
+// the sums over features (output dot, gradient, in the forward kernels' order),
+// the other the next A operand beside them; forward GEMMs start on the chunks
+// already written, and tiles alternate the accumulators so that the next tile's
+// first GEMM need not wait for the gradient sums.  1,000,003 points in FP16:
+// 801 us with one group, 757 with two, 704 with the chunks handed over.
+// Roles, waits and abort handling as in level_bf16.cuh.
 #pragma once
 
 #include "level_bf16.cuh"
@@ -29,6 +36,26 @@ namespace rgrad {
 
 using bf16::kKC;
 using bf16::kM;
+
+// compile-time flags of the drains
+struct Yes {
+  static constexpr bool value = true;
+};
+struct No {
+  static constexpr bool value = false;
+};
+
+// Warp roles: two groups of epilogue warps where they fit (32-wide units), then
+// the MMA-issuing warp and the TMA warp.
+template <int U>
+struct Roles {
+  static constexpr int kQ = 64 / U;
+  static constexpr int kGroups = U == 32 ? 2 : 1;
+  static constexpr int kEpiWarps = 4 * kQ * kGroups;
+  static constexpr int kMmaWarp = kEpiWarps;
+  static constexpr int kTmaWarp = kEpiWarps + 1;
+  static constexpr int kThreads = (kEpiWarps + 2) * 32;
+};
 
 template <int WP, int STAGES, int U>
 struct Cfg {
@@ -43,7 +70,7 @@ struct Cfg {
   static constexpr uint32_t oWout = oW0 + WP * 16;               // float [WP]
   static constexpr uint32_t oRed = oWout + WP * 4;               // float [Q-1][4][128]
   static constexpr uint32_t oBar = oRed + (Q > 1 ? Q - 1 : 1) * 4 * kM * 4;
-  static constexpr uint32_t kNumBars = 2 * STAGES + 1 + 1 + 2 + 1;
+  static constexpr uint32_t kNumBars = 2 * STAGES + bf16::kMaxNC + 1 + 1 + 2 + 1 + 1;
   static constexpr uint32_t oMisc = oBar + kNumBars * 8;
   static constexpr uint32_t oAx = (oMisc + 16 + 1023) & ~1023u;  // ones tile
   static constexpr uint32_t oBx = oAx + kM * 16 * 2;             // [nh] bias tiles
@@ -52,11 +79,12 @@ struct Cfg {
 };
 
 template <int WP, int STAGES, int U, typename T>
-__global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(const LevelArgs a) {
+__global__ void __launch_bounds__(Roles<U>::kThreads, 1) level_rgrad_kernel(const LevelArgs a) {
   using C = Cfg<WP, STAGES, U>;
-  using E = bf16::Epi<U>;
+  using E = Roles<U>;
   using Op = bf16::Operand<T>;
-  constexpr int kEpiWarps = E::kWarps;
+  constexpr int kEpiWarps = E::kEpiWarps;
+  constexpr int kGroups = E::kGroups;
   constexpr int kMmaWarp = E::kMmaWarp;
   constexpr int kTmaWarp = E::kTmaWarp;
   constexpr int kThreads = E::kThreads;
@@ -74,11 +102,13 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::oBar);
   uint64_t* wfull = bars;             // [S]  TMA -> MMA
   uint64_t* wempty = bars + S;        // [S]  MMA -> TMA
-  uint64_t* afull = bars + 2 * S;     // A operand written (count: epilogue warps)
+  uint64_t* achunk = bars + 2 * S;    // [NC] chunk of a forward GEMM's A written (count 4 Q)
+  uint64_t* afull = achunk + bf16::kMaxNC;  // a backward GEMM's A written, accumulators read
   uint64_t* dfull = afull + 1;        // GEMM done
   uint64_t* redfull = dfull + 1;      // h > 0 partials written (count 4 (Q-1))
   uint64_t* redfree = redfull + 1;    // h = 0 has read them (count 4)
-  uint64_t* finalb = redfree + 1;     // last MMA commit
+  uint64_t* gread = redfree + 1;      // B_1's accumulator read (count 4 Q)
+  uint64_t* finalb = gread + 1;       // last MMA commit
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::oMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::oMisc + 4);
   uint8_t* sAx = smem + C::oAx;
@@ -97,7 +127,9 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(
       mbar_init(&wfull[s], 1);
       mbar_init(&wempty[s], 1);
     }
+    for (int c = 0; c < bf16::kMaxNC; ++c) mbar_init(&achunk[c], 4 * Q);
     mbar_init(afull, kEpiWarps);
+    mbar_init(gread, 4 * Q);
     mbar_init(dfull, 1);
     mbar_init(redfull, 4 * (Q - 1));
     mbar_init(redfree, 4);
@@ -169,52 +201,71 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(
       const uint64_t wDesc = tc::smem_desc(smem_u32(sW), 128u, 1024u);
       const uint64_t xDesc = tc::smem_desc(smem_u32(sAx), 2048u, 128u);
       const uint64_t bxDesc = tc::smem_desc(smem_u32(sBx), 128u, 256u);
-      int64_t w = 0, k = 0;
+      int ws = 0;         // weight stage and the parity of its next fill
+      uint32_t wpar = 0;
+      uint32_t nf = 0, nb = 0, tile = 0;  // forward and backward GEMMs, tiles so far
       bool ok = true;
-      for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
-        for (int g = 0; g < G2 && ok; ++g, ++k) {
-          // GEMM k's A operand is written by drain k - 1 (or by the first
-          // layer), which has also finished with both accumulators
-          if (!bf16::mbar_wait_abort(afull, (uint32_t)(k & 1), a.status, abort_flag)) {
+      for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++tile)
+        for (int g = 0; g < G2 && ok; ++g) {
+          const bool fwd = g < nh;
+          // the second GEMM of a tile takes the accumulator of the previous
+          // tile's last one; a backward GEMM's operand is written, and its
+          // accumulator read, by the drain before it
+          if ((g == 1 && tile > 0 &&
+               !bf16::mbar_wait_abort(gread, (tile - 1) & 1, a.status, abort_flag)) ||
+              (!fwd && !bf16::mbar_wait_abort(afull, nb & 1, a.status, abort_flag))) {
             ok = false;
             break;
           }
           tc::fence_after_sync();
           const int l = layer_of(g);
-          const uint32_t d_tmem = tmem + (uint32_t)(((l - 1) & 1) * WP);
-          const bool fwd = g < nh;
+          const uint32_t d_tmem = tmem + (((uint32_t)(l - 1) ^ tile) & 1u) * WP;
           if (fwd)
             tc::mma_bf16(d_tmem, xDesc, bxDesc + (uint64_t)(((l - 1) * C::kBxBytes) >> 4), IDESC,
                          false);
-          for (int c = 0; c < NC; ++c, ++w) {
-            const int s = (int)(w % S);
-            if (!bf16::mbar_wait_abort(&wfull[s], (uint32_t)((w / S) & 1), a.status,
-                                       abort_flag)) {
+          for (int c = 0; c < NC; ++c) {
+            if ((fwd && !bf16::mbar_wait_abort(&achunk[c], nf & 1, a.status, abort_flag)) ||
+                !bf16::mbar_wait_abort(&wfull[ws], wpar, a.status, abort_flag)) {
               ok = false;
               break;
             }
             tc::fence_after_sync();
             const uint64_t aC = aDesc + (uint64_t)((c * 8 * 2048) >> 4);
-            const uint64_t wC = wDesc + (uint64_t)((s * C::kStageBytes) >> 4);
+            const uint64_t wC = wDesc + (uint64_t)((ws * C::kStageBytes) >> 4);
 #pragma unroll
             for (int ks = 0; ks < kKC / 16; ++ks)
               tc::mma_bf16(d_tmem, aC + (uint64_t)((ks * 2 * 2048) >> 4),
                            wC + (uint64_t)((ks * 256) >> 4), IDESC, fwd || c > 0 || ks > 0);
-            tc::commit(&wempty[s]);
+            tc::commit(&wempty[ws]);
+            if (++ws == S) ws = 0, wpar ^= 1u;
           }
           if (!ok) break;
           tc::commit(dfull);
+          if (fwd)
+            ++nf;
+          else
+            ++nb;
         }
       tc::commit(finalb);
       mbar_wait(finalb, 0u, a.status);
     }
   } else {
     // ================= epilogue warps =====================================
-    const int q = warp & 3, h = warp >> 2;
+    // group 0 takes what adds up over features (the output dot, the gradient),
+    // group 1 what writes the next A operand beside it; drains with one of the
+    // two are shared chunk by chunk.  One group does both.
+    const int q = warp & 3, h = (warp >> 2) % Q, grp = (warp >> 2) / Q;
+    const bool sums = grp == 0;
     const int m = 32 * q + lane;
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
     int64_t k = 0, tloc = 0;
     bool ok = true;
+    // chunk c of a forward GEMM's A operand is written by this warp
+    auto hand_chunk = [&](int c) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&achunk[c]);
+    };
     int64_t p = -1;
     float x = 0.f, y = 0.f, z = 0.f;
     {
@@ -222,11 +273,10 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(
       if (qi < n) load_point(a, qi, p, x, y, z);
     }
 #pragma unroll 1
-    for (int c = 0; c < NC; ++c)
+    for (int c = grp; c < NC; c += kGroups) {
       bf16::layer0_unit<T, false, U>(sA, w0s, WP, m, c * kKC + h * U, 0, 0.f, x, y, z);
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(afull);
+      hand_chunk(c);
+    }
     for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++tloc) {
       const int64_t tn = t + gridDim.x;
       const bool has_next = tn < ntiles;
@@ -240,58 +290,86 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(
         }
         tc::fence_after_sync();
         const int l = layer_of(g);
-        const uint32_t acc = tl + (uint32_t)(((l - 1) & 1) * WP);
+        const uint32_t flip = (uint32_t)tloc & 1u;  // tiles alternate the accumulators
+        const uint32_t acc = tl + (((uint32_t)(l - 1) ^ flip) & 1u) * WP;
         const bool last = g == G2 - 1;
         if (last && has_next) {
           const int64_t qn = tn * kM + m;
           if (qn < n) load_point(a, qn, pn, xn, yn, zn);
         }
+        // The warp's U features of a chunk go through kB at a time: with two
+        // groups a thread has 96 registers.
+        constexpr int kB = kGroups == 2 ? 16 : U;
+        auto batches = [&](int c0, int step, auto&& body, auto&& done) {
 #pragma unroll 1
-        for (int c = 0; c < NC; ++c) {
-          const int j0 = c * kKC + h * U;
-          uint32_t r[U];
-          tc::ld_32x32b<U>(acc + (uint32_t)j0, r);
-          if (g < nh - 1) {
-            // hidden forward drain: s_l = sin z_l (z_l stays in its accumulator)
-            tc::wait_ld();
-            float v[U];
+          for (int c = c0; c < NC; c += step) {
 #pragma unroll
-            for (int jj = 0; jj < U; ++jj) v[jj] = bf16::sin_fast(__uint_as_float(r[jj]));
-            bf16::store_a_unit<T, U>(sA, m, j0, v);
-          } else if (g == nh - 1) {
-            // last forward drain: the output dot and dz_nh = cos(z_nh) W_L
+            for (int b = 0; b < U; b += kB) body(c * kKC + h * U + b);
+            done(c);
+          }
+        };
+        auto nothing = [](int) {};
+        if (g < nh - 1) {
+          // hidden forward drain: s_l = sin z_l (z_l stays in its accumulator)
+          batches(grp, kGroups, [&](int j0) {
+            uint32_t r[kB];
+            tc::ld_32x32b<kB>(acc + (uint32_t)j0, r);
+            tc::wait_ld();
+            float v[kB];
+#pragma unroll
+            for (int jj = 0; jj < kB; ++jj) v[jj] = bf16::sin_fast(__uint_as_float(r[jj]));
+            bf16::store_a_unit<T, kB>(sA, m, j0, v);
+          }, hand_chunk);
+        } else if (g == nh - 1) {
+          // last forward drain: the output dot and dz_nh = cos(z_nh) W_L
+          auto both = [&](int j0, auto add, auto write) {
+            uint32_t r[kB];
+            tc::ld_32x32b<kB>(acc + (uint32_t)j0, r);
             tc::wait_ld();
             const float4* wo4 = reinterpret_cast<const float4*>(wout + j0);
-            float v[U];
+            float v[kB];
 #pragma unroll
-            for (int j4 = 0; j4 < U / 4; ++j4) {
+            for (int j4 = 0; j4 < kB / 4; ++j4) {
               const float4 wv = wo4[j4];
               const float wa[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const float zz = __uint_as_float(r[4 * j4 + i]);
-                fpart = __fmaf_rn(bf16::sin_fast(zz), wa[i], fpart);
-                v[4 * j4 + i] = __fmul_rn(__cosf(zz), wa[i]);
+                if (add.value) fpart = __fmaf_rn(bf16::sin_fast(zz), wa[i], fpart);
+                if (write.value) v[4 * j4 + i] = __fmul_rn(__cosf(zz), wa[i]);
               }
             }
-            bf16::store_a_unit<T, U>(sA, m, j0, v);
-          } else if (!last) {
-            // backward drain of B_l, l >= 2: dz_(l-1) = cos(z_(l-1)) ds_(l-1),
-            // z_(l-1) from the accumulator of G_(l-1)
-            uint32_t rz[U];
-            tc::ld_32x32b<U>(tl + (uint32_t)(((l - 2) & 1) * WP) + (uint32_t)j0, rz);
+            if (write.value) bf16::store_a_unit<T, kB>(sA, m, j0, v);
+          };
+          if (kGroups == 1)
+            batches(0, 1, [&](int j0) { both(j0, Yes(), Yes()); }, nothing);
+          else if (sums)
+            batches(0, 1, [&](int j0) { both(j0, Yes(), No()); }, nothing);
+          else
+            batches(0, 1, [&](int j0) { both(j0, No(), Yes()); }, nothing);
+        } else if (!last) {
+          // backward drain of B_l, l >= 2: dz_(l-1) = cos(z_(l-1)) ds_(l-1),
+          // z_(l-1) from the accumulator of G_(l-1)
+          batches(grp, kGroups, [&](int j0) {
+            uint32_t r[kB], rz[kB];
+            tc::ld_32x32b<kB>(acc + (uint32_t)j0, r);
+            tc::ld_32x32b<kB>(tl + (((uint32_t)(l - 2) ^ flip) & 1u) * WP + (uint32_t)j0, rz);
             tc::wait_ld();
-            float v[U];
+            float v[kB];
 #pragma unroll
-            for (int jj = 0; jj < U; ++jj)
+            for (int jj = 0; jj < kB; ++jj)
               v[jj] = __fmul_rn(__cosf(__uint_as_float(rz[jj])), __uint_as_float(r[jj]));
-            bf16::store_a_unit<T, U>(sA, m, j0, v);
-          } else {
-            // drain of B_1: dz_0 = cos(z_0) ds_0 with z_0 recomputed in FP32,
-            // df/dx = (w0 W0)^T dz_0
+            bf16::store_a_unit<T, kB>(sA, m, j0, v);
+          }, nothing);
+        } else {
+          // drain of B_1: dz_0 = cos(z_0) ds_0 with z_0 recomputed in FP32,
+          // df/dx = (w0 W0)^T dz_0; and the next tile's first layer
+          auto gradient = [&](int j0) {
+            uint32_t r[kB];
+            tc::ld_32x32b<kB>(acc + (uint32_t)j0, r);
             tc::wait_ld();
 #pragma unroll
-            for (int j4 = 0; j4 < U / 4; ++j4) {
+            for (int j4 = 0; j4 < kB / 4; ++j4) {
               float zz[4];
               float4 wx, wy, wz;
               bf16::phase4(w0s, WP, j0 + 4 * j4, x, y, z, zz, wx, wy, wz);
@@ -306,22 +384,36 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) level_rgrad_kernel(
                 g2 = __fmaf_rn(dz, az[i], g2);
               }
             }
-            if (has_next)
-              bf16::layer0_unit<T, false, U>(sA, w0s, WP, m, j0, 0, 0.f, xn, yn, zn);
-          }
+          };
+          auto first = [&](int j0) {
+            bf16::layer0_unit<T, false, kB>(sA, w0s, WP, m, j0, 0, 0.f, xn, yn, zn);
+          };
+          if (kGroups == 1)
+            batches(0, 1, [&](int j0) {
+              gradient(j0);
+              if (has_next) first(j0);
+            }, [&](int c) { if (has_next) hand_chunk(c); });
+          else if (sums)
+            batches(0, 1, gradient, nothing);
+          else if (has_next)
+            batches(0, 1, first, hand_chunk);
         }
-        // this drain wrote the A operand of the next GEMM (of this tile, or
-        // the next tile's first); the accumulators are free for it
-        const bool hand_over = !last || has_next;
-        if (hand_over) fence_proxy_async_smem();
+        // a backward GEMM follows: its whole A operand is written and the
+        // accumulator it overwrites is read; or the tile's last accumulator is
+        const bool to_backward = g >= nh - 1 && !last;
+        if (to_backward) fence_proxy_async_smem();
         tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0 && hand_over) mbar_arrive(afull);
+        if (lane == 0) {
+          if (to_backward) mbar_arrive(afull);
+          if (last && sums) mbar_arrive(gread);
+        }
       }
       if (!ok) break;
 
       // combine the feature splits: f, df/dx, df/dy, df/dz of each point
-      if (h > 0) {
+      if (!sums) {
+      } else if (h > 0) {
         if (tloc >= 1 && !bf16::warp_wait(redfree, (uint32_t)((tloc - 1) & 1), a.status,
                                           abort_flag)) {
           ok = false;
@@ -383,7 +475,7 @@ int launch_cfg(const LevelArgs& a, cudaStream_t s) {
     grid = ntiles < grid ? ntiles : grid;
   }
   if (grid <= 0) return MPL_OK;
-  level_rgrad_kernel<WP, STAGES, U, T><<<(unsigned)grid, bf16::Epi<U>::kThreads, smem, s>>>(a);
+  level_rgrad_kernel<WP, STAGES, U, T><<<(unsigned)grid, Roles<U>::kThreads, smem, s>>>(a);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
 }
