@@ -339,18 +339,36 @@ int launch_wgrad(const TrainArgs& t, int WP, const WgradOut& out, cudaStream_t s
 
 // Layer 0 (3 inputs): dW0[j][c] += sum_q da_v[j] x_qc + da_tc[j]; db0[j] += da_v[j].
 // Output layer: dWL[j] += sum_rows seed_row out_(L-1)[row][j]; dbL += seed_v.
-// Thread j of a block, 8 points per step; each block covers a contiguous
-// point range and adds its partial sums atomically.
+// Thread j of a block, four points' loads in flight; each block covers a
+// contiguous point range and adds its partial sums atomically.  dbL, a sum of
+// signed seeds that mostly cancel, is one block's (the last), in double: its
+// float partial sums in atomic order moved it by 1e-6 from run to run.
+// Bound: the latency of the rows' loads (15,000 points 76 -> 59 us).
 __global__ void __launch_bounds__(256) train_wgrad_ends_kernel(const TrainArgs a, int WP,
                                                                float* dW0, float* db0, float* dWL,
                                                                float* dbL) {
   const int nh = a.lay.nh;
-  const int64_t per = (a.n + gridDim.x - 1) / gridDim.x;
+  if (blockIdx.x == gridDim.x - 1) {
+    double b = 0.0;
+    for (int64_t q = threadIdx.x; q < a.n; q += blockDim.x) b += (double)a.seed[q * 4];
+    for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+    __shared__ double part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = b;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b += part[w];
+      atomicAdd(dbL, (float)b);
+    }
+    return;
+  }
+  const int64_t nb = gridDim.x - 1;
+  const int64_t per = (a.n + nb - 1) / nb;
   const int64_t q_begin = blockIdx.x * per;
   const int64_t q_end = q_begin + per < a.n ? q_begin + per : a.n;
   const float om = a.omega[nh];
   for (int j = threadIdx.x; j < WP; j += blockDim.x) {
     float w0x = 0.f, w0y = 0.f, w0z = 0.f, b0 = 0.f, wl = 0.f;
+#pragma unroll 4
     for (int64_t q = q_begin; q < q_end; ++q) {
       const float* d = a.da + (q * 4) * WP;  // layer 0
       const float dv = d[j];
@@ -373,11 +391,6 @@ __global__ void __launch_bounds__(256) train_wgrad_ends_kernel(const TrainArgs a
     atomicAdd(&dW0[j * 3 + 2], w0z);
     atomicAdd(&db0[j], b0);
     atomicAdd(&dWL[j], wl);
-  }
-  if (threadIdx.x == 0) {
-    float b = 0.f;
-    for (int64_t q = q_begin; q < q_end; ++q) b = __fadd_rn(b, a.seed[q * 4]);
-    atomicAdd(dbL, b);
   }
 }
 
@@ -610,9 +623,9 @@ extern "C" int mpl_train_backward(const MplNet* net, const void* packed, const f
     st = WP == 64 ? launch_wgrad<64>(t, WP, out, s) : launch_wgrad<128>(t, WP, out, s);
     if (st != MPL_OK) return st;
   }
-  // about 64 points per block
-  const int64_t eb = (n + 63) / 64 < 4096 ? (n + 63) / 64 : 4096;
-  train_wgrad_ends_kernel<<<(unsigned)eb, WP < 256 ? WP : 256, 0, s>>>(t, WP, dW[0], db[0],
+  // 16 points a block, up to 4096 blocks, and the one of dbL
+  const int64_t eb = (n + 15) / 16 < 4096 ? (n + 15) / 16 : 4096;
+  train_wgrad_ends_kernel<<<(unsigned)(eb + 1), WP < 256 ? WP : 256, 0, s>>>(t, WP, dW[0], db[0],
                                                                        dW[L - 1], db[L - 1]);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
