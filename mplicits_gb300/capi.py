@@ -194,6 +194,8 @@ class MplError(RuntimeError):
 def load(path=LIB_PATH):
     """Load libmplicits.so (raises if it is missing: there is no fallback)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(path):
@@ -222,9 +224,13 @@ def check(status, where):
 
 
 def stream_ptr(stream=None):
+    """The CUDA stream handle of ``stream``, or of the current device's current
+    stream (asked for as the raw handle: no Stream object per call)."""
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    return ctypes.c_void_p(
+        torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t):

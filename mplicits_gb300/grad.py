@@ -40,29 +40,18 @@ def level_gradient(model, x, S=None, G=None, accumulate=False, precision=None, i
     return S, G
 
 
-def level_backward(model, x, gy, params, needs_input_grad):
-    """Backward of model_out = f(x) for ``_LevelForward``.
+def level_backward(model, x, gy):
+    """d(model_in) of model_out = f(x) for ``_LevelForward``: gy * df/dx.
 
-    d(model_in) = gy * df/dx comes from the fused gradient kernel; under
-    ``create_graph=True`` (i3d/diff_operators.py:259-265) it is the
-    differentiable op of ``mplicits_gb300.train.level_input_grad``, whose own
-    backward is the double backward of the eikonal and normal losses.
-    Weight gradients come from the hand-written backward kernels
-    (``mplicits_gb300.train.param_grads``) with seed gy.
+    It comes from the fused gradient kernel; under ``create_graph=True``
+    (i3d/diff_operators.py:259-265) df/dx is the differentiable op of
+    ``mplicits_gb300.train.level_input_grad``, whose own backward is the double
+    backward of the eikonal and normal losses.
     """
     from . import train as _train
     shape = x.shape
-    x2 = x.detach().reshape(-1, shape[-1])
-    g2 = gy.reshape(-1)
-    dx = None
-    if needs_input_grad[0]:
-        if torch.is_grad_enabled():
-            G = _train.level_input_grad(model, x.reshape(-1, shape[-1]))
-            dx = (gy.reshape(-1, 1) * G).reshape(shape)
-        else:
-            _, G = level_gradient(model, x2, precision="fp32")
-            dx = (g2.reshape(-1, 1).to(G.dtype) * G).reshape(shape)
-    pgrads = (None,) * len(params)
-    if any(needs_input_grad[2:]):
-        pgrads = tuple(_train.param_grads(model, x2, df=g2.detach()))
-    return (dx, None) + pgrads
+    if torch.is_grad_enabled():
+        G = _train.level_input_grad(model, x.reshape(-1, shape[-1]))
+        return (gy.reshape(-1, 1) * G).reshape(shape)
+    _, G = level_gradient(model, x.detach().reshape(-1, shape[-1]), precision="fp32")
+    return (gy.reshape(-1, 1).to(G.dtype) * G).reshape(shape)

@@ -62,9 +62,18 @@ class PackedLevel:
         self.net = None
 
     def get(self, model):
-        params = [p for p in model.parameters()]
-        key = tuple((p.data_ptr(), p._version) for p in params) + \
-            (model.w0, model.ww, params[0].device)
+        lins = model.linears()
+        first = lins[0].weight
+        key = [model.w0, model.ww, first.device]
+        for lin in lins:
+            own = lin._parameters  # a plain lookup where nothing is parametrized
+            for p in (own.get("weight"), own.get("bias")):
+                if p is None:
+                    key += [p.data_ptr() for p in (lin.weight, lin.bias)]
+                    key += [p._version for p in (lin.weight, lin.bias)]
+                    break
+                key.append(p.data_ptr())
+                key.append(p._version)
         if key == self.key:
             return self.net, self.buf
         net = model.mpl_net()
@@ -72,12 +81,12 @@ class PackedLevel:
         nbytes = ctypes.c_int64(0)
         capi.check(lib.mpl_net_packed_bytes(ctypes.byref(net), ctypes.byref(nbytes)),
                    "mpl_net_packed_bytes")
-        dev = params[0].device
+        dev = first.device
         buf = torch.empty(nbytes.value + 256, dtype=torch.uint8, device=dev)
         off = (-buf.data_ptr()) % 256
         view = buf[off:off + nbytes.value]
-        ws = [l.weight.detach().contiguous().float() for l in model.linears()]
-        bs = [l.bias.detach().contiguous().float() for l in model.linears()]
+        ws = [l.weight.detach().contiguous().float() for l in lins]
+        bs = [l.bias.detach().contiguous().float() for l in lins]
         wp = (ctypes.c_void_p * len(ws))(*[w.data_ptr() for w in ws])
         bp = (ctypes.c_void_p * len(bs))(*[b.data_ptr() for b in bs])
         capi.check(lib.mpl_net_pack(ctypes.byref(net), wp, bp, capi.ptr(view),
@@ -94,8 +103,9 @@ def _require_cuda(x):
 
 
 class _LevelForward(torch.autograd.Function):
-    """model_out = f(x) through mpl_level_forward; backward via the
-    input-gradient and weight-gradient kernels (see mplicits_gb300.grad)."""
+    """model_out = f(x) through mpl_level_forward; its backward gives d(x) by
+    the input-gradient kernel (see mplicits_gb300.grad), and no parameter
+    gradients: those are ``_LevelParams``'s."""
 
     @staticmethod
     def forward(ctx, x, model, *params):
@@ -108,17 +118,37 @@ class _LevelForward(torch.autograd.Function):
     def backward(ctx, gy):
         from . import grad as _grad
         x, *params = ctx.saved_tensors
-        return _grad.level_backward(ctx.model, x, gy, params, ctx.needs_input_grad)
+        dx = _grad.level_backward(ctx.model, x, gy) if ctx.needs_input_grad[0] else None
+        return (dx, None) + (None,) * len(params)
+
+
+class _LevelParams(torch.autograd.Function):
+    """Zeros whose backward gives the level's parameter gradients (the
+    weight-gradient kernels).  Added to model_out as a node of its own, so that
+    autograd runs it only when a parameter's gradient is asked for: a Function
+    cannot tell that ``torch.autograd.grad(model_out, model_in)`` wants none."""
+
+    @staticmethod
+    def forward(ctx, x, model, *params):
+        ctx.model = model
+        ctx.save_for_backward(x, *params)
+        return torch.zeros(x.shape[:-1] + (1,), dtype=torch.float32, device=x.device)
+
+    @staticmethod
+    def backward(ctx, gy):
+        from . import train as _train
+        x, *params = ctx.saved_tensors
+        grads = _train.param_grads(ctx.model, x.reshape(-1, x.shape[-1]),
+                                   df=gy.detach().reshape(-1))
+        return (None, None) + tuple(grads)
 
 
 def level_forward(model, x, S=None, accumulate=False, precision=None):
     """One launch of the fused level kernel on points ``x`` [P, 3]; returns
     (or accumulates into) ``S`` [P]."""
     _require_cuda(x)
-    x = x.detach()
-    if x.dtype != torch.float32:
-        x = x.float()
-    x = x.contiguous()
+    if x.dtype != torch.float32 or not x.is_contiguous():
+        x = x.detach().float().contiguous()
     P = x.shape[0]
     if S is None:
         S = torch.empty(P, dtype=torch.float32, device=x.device)
@@ -159,7 +189,7 @@ class SIREN(nn.Module):
 
     # -- topology --------------------------------------------------------
     def linears(self):
-        return [blk[0] for blk in self.net]
+        return [blk._modules["0"] for blk in self._modules["net"]._modules.values()]
 
     def omegas(self):
         out = []
@@ -189,13 +219,16 @@ class SIREN(nn.Module):
     def forward(self, x, preserve_grad=False):
         """Same contract as i3d/model.py:107-129."""
         coords_org = x if preserve_grad else x.clone().detach().requires_grad_(True)
-        params = tuple(self.parameters())
-        if torch.is_grad_enabled() and (coords_org.requires_grad or
-                                        any(p.requires_grad for p in params)):
-            y = _LevelForward.apply(coords_org, self, *params)
-        else:
-            y = level_forward(self, coords_org.reshape(-1, coords_org.shape[-1]))
-            y = y.reshape(coords_org.shape[:-1] + (1,))
+        if torch.is_grad_enabled():
+            params = tuple(self.parameters())
+            trained = any(p.requires_grad for p in params)
+            if coords_org.requires_grad or trained:
+                y = _LevelForward.apply(coords_org, self, *params)
+                if trained:
+                    y = y + _LevelParams.apply(coords_org.detach(), self, *params)
+                return {"model_in": coords_org, "model_out": y}
+        y = level_forward(self, coords_org.reshape(-1, coords_org.shape[-1]))
+        y = y.reshape(coords_org.shape[:-1] + (1,))
         return {"model_in": coords_org, "model_out": y}
 
     def reset_weights(self):

@@ -18,6 +18,7 @@ followed by ``loss.backward()`` (the reference trainers' own code) trains a
 from __future__ import annotations
 
 import ctypes
+import math
 
 import torch
 
@@ -51,19 +52,30 @@ class _Scratch:
         self.g = torch.empty(n, 3, dtype=torch.float32, device=device)
         self.seeds = torch.empty(n, 4, dtype=torch.float32, device=device)
         self.n = n
-        # padded gradient buffers, one per nn.Linear weight and bias
+        # padded gradient buffers, one per nn.Linear weight and bias, in one
+        # allocation (zeroed and copied by one launch each), every part at a
+        # multiple of 256 bytes
         wp = _padded_width(self.model)
-        L = len(self.model.linears())
-        self.dW, self.db = [], []
+        lins = self.model.linears()
+        L = len(lins)
+        self.shapes = []
         for l in range(L):
-            rows = wp if l < L - 1 else 1
-            cols = 3 if l == 0 else wp
-            if l == L - 1:
-                self.dW.append(torch.zeros(wp, dtype=torch.float32, device=device))
-                self.db.append(torch.zeros(1, dtype=torch.float32, device=device))
-            else:
-                self.dW.append(torch.zeros(rows, cols, dtype=torch.float32, device=device))
-                self.db.append(torch.zeros(wp, dtype=torch.float32, device=device))
+            self.shapes += [(1, wp), (1,)] if l == L - 1 else \
+                [(wp, 3 if l == 0 else wp), (wp,)]
+        self.starts, at = [], 0
+        for s in self.shapes:
+            self.starts.append(at)
+            at += (math.prod(s) + 63) // 64 * 64
+        self.flat = torch.zeros(at, dtype=torch.float32, device=device)
+        parts = self.parts(self.flat)
+        self.dW, self.db = parts[0::2], parts[1::2]
+        # whether the parameters have exactly the padded shapes
+        self.exact = all(tuple(p.shape) == s for l in range(L) for p, s in zip(
+            (lins[l].weight, lins[l].bias), self.shapes[2 * l:2 * l + 2]))
+
+    def parts(self, flat):
+        """The views of a flat gradient buffer, weight and bias per layer."""
+        return [flat[a:a + math.prod(s)].view(s) for a, s in zip(self.starts, self.shapes)]
 
 
 def _padded_width(model):
@@ -91,8 +103,7 @@ def _forward_with_scratch(model, x, sc):
 def _backward(model, x, sc):
     """Weight gradients into the padded buffers (zeroed first)."""
     net, packed = model.packed()
-    for t in sc.dW + sc.db:
-        t.zero_()
+    sc.flat.zero_()
     n = x.shape[0]
     dW = (ctypes.c_void_p * len(sc.dW))(*[t.data_ptr() for t in sc.dW])
     db = (ctypes.c_void_p * len(sc.db))(*[t.data_ptr() for t in sc.db])
@@ -101,17 +112,16 @@ def _backward(model, x, sc):
         capi.ptr(sc.seeds[:n]), capi.ptr(sc.da), dW, db, capi.stream_ptr()), "mpl_train_backward")
 
 
-def _unpad(model, sc):
-    """Gradients in the shapes of the nn.Linear parameters (weight, bias, ...)."""
+def _unpad(model, sc, own=True):
+    """Gradients in the shapes of the nn.Linear parameters (weight, bias, ...):
+    tensors of the caller's, or with ``own=False`` views that the next backward
+    overwrites where no padding has to be cut off."""
+    if sc.exact:
+        return sc.parts(sc.flat.clone() if own else sc.flat)
     out = []
-    L = len(model.linears())
     for l, lin in enumerate(model.linears()):
-        if l == L - 1:
-            out.append(sc.dW[l][:lin.in_features].reshape(1, -1).clone())
-            out.append(sc.db[l][:1].clone())
-        else:
-            out.append(sc.dW[l][:lin.out_features, :lin.in_features].clone())
-            out.append(sc.db[l][:lin.out_features].clone())
+        out.append(sc.dW[l][:lin.out_features, :lin.in_features].clone())
+        out.append(sc.db[l][:lin.out_features].clone())
     return out
 
 
@@ -242,6 +252,7 @@ class ResidualTrainer:
         self.exp_avg_sq = [torch.zeros_like(p) for p in self.params]
         self.t = 0
         self.loss_sums = torch.zeros(4, dtype=torch.float32, device=self.params[0].device)
+        self._scale_n = None  # (n, scale / n) of the last batch size
         self._scale = torch.tensor([w[k] for k in self.names], dtype=torch.float32,
                                    device=self.params[0].device)
 
@@ -249,6 +260,15 @@ class ResidualTrainer:
     def loss_and_grads(self, x, normals, sdf):
         """The weighted loss terms (``self.names``) and the gradients of their
         sum, in ``model.parameters()`` order."""
+        return self._loss_and_grads(x, normals, sdf, own=True)
+
+    def _terms(self, n):
+        """The weighted loss terms from the sums over n points."""
+        if self._scale_n is None or self._scale_n[0] != n:
+            self._scale_n = (n, self._scale / n)
+        return self.loss_sums[:len(self.names)] * self._scale_n[1]
+
+    def _loss_and_grads(self, x, normals, sdf, own):
         x = x.detach().float().reshape(-1, 3).contiguous()
         normals = normals.detach().float().reshape(-1, 3).contiguous()
         sdf = sdf.detach().float().reshape(-1).contiguous()
@@ -260,7 +280,7 @@ class ResidualTrainer:
             for i, m in enumerate(self.frozen):
                 level_gradient(m, x, S=Ff, G=Gf, accumulate=i > 0, precision=self.precision)
         if self.precision == "bf16":
-            return self._tc_loss_and_grads(x, normals, sdf, Ff, Gf)
+            return self._tc_loss_and_grads(x, normals, sdf, Ff, Gf, own)
         sc = _scratch(self.model, n, x.device)
         _forward_with_scratch(self.model, x, sc)
         capi.check(capi.load().mpl_train_loss(
@@ -268,10 +288,9 @@ class ResidualTrainer:
             capi.ptr(normals), ctypes.byref(self.loss), capi.ptr(sc.seeds[:n]),
             capi.ptr(self.loss_sums), capi.stream_ptr()), "mpl_train_loss")
         _backward(self.model, x, sc)
-        grads = _unpad(self.model, sc)
-        return self.loss_sums[:len(self.names)] * (self._scale / n), grads
+        return self._terms(n), _unpad(self.model, sc, own)
 
-    def _tc_loss_and_grads(self, x, normals, sdf, Ff, Gf):
+    def _tc_loss_and_grads(self, x, normals, sdf, Ff, Gf, own):
         """One mpl_train_tc_step: forward, loss, backward and weight gradients
         on the tensor cores."""
         n = x.shape[0]
@@ -290,8 +309,7 @@ class ResidualTrainer:
         if seeds is None or seeds.shape[0] < n:
             seeds = torch.empty(n, 4, dtype=torch.float32, device=x.device)
             self._tc_seeds = seeds
-        for t in sc.dW + sc.db:
-            t.zero_()
+        sc.flat.zero_()
         P = ctypes.c_void_p
         dW = (P * len(sc.dW))(*[t.data_ptr() for t in sc.dW])
         db = (P * len(sc.db))(*[t.data_ptr() for t in sc.db])
@@ -300,12 +318,11 @@ class ResidualTrainer:
             capi.ptr(sdf), capi.ptr(normals), ctypes.byref(self.loss),
             ctypes.c_void_p(buf.data_ptr() + off), nb.value, capi.ptr(seeds),
             capi.ptr(self.loss_sums), dW, db, capi.stream_ptr()), "mpl_train_tc_step")
-        grads = _unpad(self.model, sc)
-        return self.loss_sums[:len(self.names)] * (self._scale / n), grads
+        return self._terms(n), _unpad(self.model, sc, own)
 
     @torch.no_grad()
     def step(self, x, normals, sdf):
-        losses, grads = self.loss_and_grads(x, normals, sdf)
+        losses, grads = self._loss_and_grads(x, normals, sdf, own=False)
         self.t += 1
         cnt = len(self.params)
         P = ctypes.c_void_p
