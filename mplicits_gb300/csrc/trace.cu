@@ -14,6 +14,8 @@ namespace mpl {
 
 namespace {
 
+constexpr int kThreads = 256;
+
 struct Basis {
   float eye[3], s[3], u[3], f[3];
   float tx, ty;  // tan(fov/2) * aspect, tan(fov/2)
@@ -28,10 +30,10 @@ __global__ void trace_init_kernel(Basis b, int W, int H, float R, float* __restr
                                   float* __restrict__ dir, int32_t* __restrict__ state,
                                   int32_t* __restrict__ active, int32_t* __restrict__ count) {
   const int64_t P = (int64_t)W * H;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~int64_t(31);
-  for (int64_t base = warp0; base < P; base += stride) {
-    const int64_t r = base + (threadIdx.x & 31);
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  int turn = 0;
+  for (int64_t base = (int64_t)blockIdx.x * kThreads; base < P; base += stride, ++turn) {
+    const int64_t r = base + threadIdx.x;
     bool keep = false;
     if (r < P) {
       const int i = (int)(r % W), j = (int)(r / W);
@@ -62,7 +64,7 @@ __global__ void trace_init_kernel(Basis b, int W, int H, float R, float* __restr
       state[r] = hits_sphere ? 0 : 2;
       keep = hits_sphere;
     }
-    warp_append(keep, (int32_t)r, active, count, P);
+    block_append<1, kThreads>(turn, {keep}, (int32_t)r, {active}, {count}, P);
   }
 }
 
@@ -80,10 +82,10 @@ __global__ void trace_step_kernel(const float* __restrict__ S, const int32_t* __
                                   int64_t capacity) {
   int64_t n = *count;
   n = n < cap_in ? n : cap_in;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~int64_t(31);
-  for (int64_t base = warp0; base < n; base += stride) {
-    const int64_t q = base + (threadIdx.x & 31);
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  int turn = 0;
+  for (int64_t base = (int64_t)blockIdx.x * kThreads; base < n; base += stride, ++turn) {
+    const int64_t q = base + threadIdx.x;
     bool keep = false, hit = false;
     int32_t r = 0;
     if (q < n) {
@@ -92,8 +94,8 @@ __global__ void trace_step_kernel(const float* __restrict__ S, const int32_t* __
       hit = st == 1;
       keep = st == 0;
     }
-    warp_append(keep, r, active_out, count_out, capacity);
-    warp_append(hit, r, hit_out, hit_count, capacity);
+    block_append<2, kThreads>(turn, {keep, hit}, r, {active_out, hit_out},
+                              {count_out, hit_count}, capacity);
   }
 }
 
@@ -177,7 +179,7 @@ extern "C" int mpl_trace_init(const MplCamera* cam, float radius, float* origins
   MPL_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(int32_t), s));
   int64_t blocks = (P + 255) / 256;
   if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-  trace_init_kernel<<<(unsigned)blocks, 256, 0, s>>>(make_basis(*cam), cam->width, cam->height,
+  trace_init_kernel<<<(unsigned)blocks, kThreads, 0, s>>>(make_basis(*cam), cam->width, cam->height,
                                                      radius, origins, dirs, state, active, count);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
@@ -196,7 +198,7 @@ extern "C" int mpl_trace_step(const float* S, const int32_t* active, const int32
   if (n_max == 0) return MPL_OK;
   int64_t blocks = (n_max + 255) / 256;
   if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-  trace_step_kernel<<<(unsigned)blocks, 256, 0, s>>>(S, active, count, n_max, origins, dirs,
+  trace_step_kernel<<<(unsigned)blocks, kThreads, 0, s>>>(S, active, count, n_max, origins, dirs,
                                                      state, eps, radius, last_step, active_out,
                                                      count_out, hit_out, hit_count, capacity);
   MPL_LAUNCH_CHECK();
