@@ -12,17 +12,23 @@
 // kernel (FP32 first layer and sines, 16-bit GEMM operands, the same output
 // reduction) and of trace_step_kernel, so a frame gives the same image.
 //
-// Roles (as the level kernels): 4*Q epilogue warps, one MMA-issuing warp,
-// one TMA warp.  One accumulator and one A operand: GEMM k waits for its A
-// operand (afull, written by the first layer or by the previous drain) and
-// for the previous accumulator to be drained (dempty); the epilogue waits for
-// dfull.  The weights of every level stream through one ring in the MMA's
-// GEMM order (tile, step, level, layer).  The first layer of level l + 1 is
-// written inside the last drain of level l (the rays have not moved).  The
-// epilogue warps meet at a named barrier twice per step, once with every
-// level's feature-split partial sums written and once after the marching
-// step; its reduction carries the abort decision, so all of them leave
-// together.
+// Roles: two groups of 4*Q epilogue warps (one at 16-wide units), one
+// MMA-issuing warp, one TMA warp.  A CTA has one tile, so a step lasts as long
+// as its chain of GEMMs and drains; the chain is kept short:
+//   - hidden drains are shared by the groups chunk by chunk; in a level's last
+//     drain group 0 takes the output dot while group 1 writes the first layer of
+//     the next level (the rays have not moved);
+//   - the two accumulators alternate, so a GEMM starts on the A chunks already
+//     written (achunk) while the drain before it still reads the other one.
+// GEMM k waits for its chunks and for the drain of GEMM k - 2 (dempty); the
+// epilogue waits for dfull, one barrier per accumulator, because group 0 may
+// still be in drain k when GEMM k + 1 is done.  The weights of every level
+// stream through one ring in the MMA's GEMM order (tile, step, level, layer).
+// The epilogue warps meet at a named barrier twice per step, once with every
+// level's feature-split partial sums written and once after the marching step;
+// its reduction carries the abort decision, so all of them leave together.
+// Bound: that chain's latency.  64 steps of a full-HD frame's last rays, three
+// 256-wide levels: 1385 us with one group and one accumulator, 1135 now.
 // Every mbarrier wait is bounded (the abort protocol of level_bf16.cuh).
 #include <string.h>
 
@@ -60,6 +66,16 @@ struct Args {
   int* status;
 };
 
+template <int U>
+struct Roles {
+  static constexpr int kQ = 64 / U;
+  static constexpr int kGroups = U == 32 ? 2 : 1;
+  static constexpr int kEpiWarps = 4 * kQ * kGroups;
+  static constexpr int kMmaWarp = kEpiWarps;
+  static constexpr int kTmaWarp = kEpiWarps + 1;
+  static constexpr int kThreads = (kEpiWarps + 2) * 32;
+};
+
 template <int WP, int U>
 struct Cfg {
   static constexpr int NC = WP / kKC;
@@ -73,7 +89,7 @@ struct Cfg {
   static constexpr uint32_t oRed = oWout + kMaxLevels * WP * 4;        // float [levels][Q][128]
   static constexpr uint32_t oPos = oRed + kMaxLevels * Q * kM * 4;    // float4 [128] x, y, z, alive
   static constexpr uint32_t oBar = oPos + kM * 16;
-  static constexpr uint32_t kNumBars = 2 * kStages + 4;
+  static constexpr uint32_t kNumBars = 2 * kStages + bf16::kMaxNC + 5;
   static constexpr uint32_t oMisc = oBar + kNumBars * 8;              // tmem slot, abort, bout[3]
   // the biases of every hidden layer j = level * nh + layer - 1 share one
   // bias tile (K columns 2j, 2j + 1: the two 16-bit pieces of omega*b); the
@@ -87,11 +103,12 @@ struct Cfg {
 };
 
 template <int WP, int U, typename T>
-__global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) trace_march_kernel(const Args a) {
+__global__ void __launch_bounds__(Roles<U>::kThreads, 1) trace_march_kernel(const Args a) {
   using C = Cfg<WP, U>;
-  using E = bf16::Epi<U>;
+  using E = Roles<U>;
   using Op = bf16::Operand<T>;
-  constexpr int kEpiWarps = E::kWarps;
+  constexpr int kEpiWarps = E::kEpiWarps;
+  constexpr int kGroups = E::kGroups;
   constexpr int kMmaWarp = E::kMmaWarp;
   constexpr int kTmaWarp = E::kTmaWarp;
   constexpr int kThreads = E::kThreads;
@@ -110,10 +127,10 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) trace_march_kernel(
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::oBar);
   uint64_t* wfull = bars;           // [S]  TMA -> MMA
   uint64_t* wempty = bars + S;      // [S]  MMA -> TMA
-  uint64_t* afull = bars + 2 * S;   // A operand written (count: epilogue warps)
-  uint64_t* dfull = afull + 1;      // accumulator ready
-  uint64_t* dempty = dfull + 1;     // accumulator drained (count: epilogue warps)
-  uint64_t* finalb = dempty + 1;    // last MMA commit
+  uint64_t* achunk = bars + 2 * S;  // [NC] A chunk written (count 4 Q: one group)
+  uint64_t* dfull = achunk + bf16::kMaxNC;  // [2] accumulator ready
+  uint64_t* dempty = dfull + 2;     // [2] accumulator drained (count: epilogue warps)
+  uint64_t* finalb = dempty + 2;    // last MMA commit
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::oMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::oMisc + 4);
   float* bouts = reinterpret_cast<float*>(smem + C::oMisc + 8);  // [levels] output biases
@@ -136,14 +153,16 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) trace_march_kernel(
       mbar_init(&wfull[s], 1);
       mbar_init(&wempty[s], 1);
     }
-    mbar_init(afull, kEpiWarps);
-    mbar_init(dfull, 1);
-    mbar_init(dempty, kEpiWarps);
+    for (int c = 0; c < bf16::kMaxNC; ++c) mbar_init(&achunk[c], 4 * Q);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&dfull[b], 1);
+      mbar_init(&dempty[b], kEpiWarps);
+    }
     mbar_init(finalb, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == kMmaWarp) tc::tmem_alloc(tmem_slot, WP);
+  if (warp == kMmaWarp) tc::tmem_alloc(tmem_slot, 2 * WP);
   for (int lev = 0; lev < L; ++lev) {
     const char* pk = a.packed[lev];
     const PackLayout& lay = a.lay[lev];
@@ -214,60 +233,69 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) trace_march_kernel(
       const uint64_t wDesc = tc::smem_desc(smem_u32(sW), 128u, 1024u);
       const uint64_t xDesc = tc::smem_desc(smem_u32(sAx), 2048u, 128u);
       const uint64_t bxDesc = tc::smem_desc(smem_u32(sBx), 128u, 256u);
-      int64_t w = 0, k = 0;
+      int ws = 0;  // weight stage and the parity of its next fill
+      uint32_t wpar = 0, k = 0;
       bool ok = true;
       for (int64_t t = blockIdx.x; t < ntiles && ok; t += G)
         for (int st = 0; st < a.steps && ok; ++st)
           for (int lev = 0; lev < L && ok; ++lev)
             for (int l = 1; l <= nh && ok; ++l, ++k) {
-              if ((k > 0 && !bf16::mbar_wait_abort(dempty, (uint32_t)((k - 1) & 1), a.status,
-                                                   abort_flag)) ||
-                  !bf16::mbar_wait_abort(afull, (uint32_t)(k & 1), a.status, abort_flag)) {
+              const uint32_t b = k & 1u;
+              if (k >= 2 && !bf16::mbar_wait_abort(&dempty[b], ((k >> 1) - 1) & 1u, a.status,
+                                                   abort_flag)) {
                 ok = false;
                 break;
               }
               tc::fence_after_sync();
-              tc::mma_bf16(tmem, xDesc + (uint64_t)(((lev * nh + l - 1) * C::kOnesBytes) >> 4),
+              const uint32_t d_tmem = tmem + b * WP;
+              tc::mma_bf16(d_tmem, xDesc + (uint64_t)(((lev * nh + l - 1) * C::kOnesBytes) >> 4),
                            bxDesc, IDESC, false);
-              for (int c = 0; c < NC; ++c, ++w) {
-                const int s = (int)(w % S);
-                if (!bf16::mbar_wait_abort(&wfull[s], (uint32_t)((w / S) & 1), a.status,
-                                           abort_flag)) {
+              for (int c = 0; c < NC; ++c) {
+                if (!bf16::mbar_wait_abort(&achunk[c], k & 1u, a.status, abort_flag) ||
+                    !bf16::mbar_wait_abort(&wfull[ws], wpar, a.status, abort_flag)) {
                   ok = false;
                   break;
                 }
                 tc::fence_after_sync();
                 const uint64_t aC = aDesc + (uint64_t)((c * 8 * 2048) >> 4);
-                const uint64_t wC = wDesc + (uint64_t)((s * C::kStageBytes) >> 4);
+                const uint64_t wC = wDesc + (uint64_t)((ws * C::kStageBytes) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < kKC / 16; ++ks)
-                  tc::mma_bf16(tmem, aC + (uint64_t)((ks * 2 * 2048) >> 4),
+                  tc::mma_bf16(d_tmem, aC + (uint64_t)((ks * 2 * 2048) >> 4),
                                wC + (uint64_t)((ks * 256) >> 4), IDESC, true);
-                tc::commit(&wempty[s]);
+                tc::commit(&wempty[ws]);
+                if (++ws == S) ws = 0, wpar ^= 1u;
               }
               if (!ok) break;
-              tc::commit(dfull);
+              tc::commit(&dfull[b]);
             }
       tc::commit(finalb);
       mbar_wait(finalb, 0u, a.status);
     }
   } else {
     // ================= epilogue warps =====================================
-    const int q = warp & 3, h = warp >> 2;
+    const int q = warp & 3, h = (warp >> 2) % Q, grp = (warp >> 2) / Q;
+    const bool sums = grp == 0, firsts = grp == kGroups - 1;
+    const bool own = sums && h == 0;  // the warps that own the tile's rays
     const int m = 32 * q + lane;
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
     constexpr int kEpiThreads = kEpiWarps * 32;
-    int64_t k = 0;  // GEMMs drained
+    uint32_t k = 0;  // GEMMs drained
+    auto hand_chunk = [&](int c) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&achunk[c]);
+    };
     bool fail = false;
     for (int64_t t = blockIdx.x; t < ntiles && !fail; t += G) {
       const int64_t qi = t * kM + m;
       const int64_t r = qi < n ? (int64_t)a.active[qi] : -1;
-      // the h = 0 warps own the tile's rays: position, direction and state in
+      // the h = 0 warps of group 0 own the tile's rays: position, direction and state in
       // registers, the position shared with the other warps through smem;
       // the frame's arrays are written when a ray stops
       float o[3] = {0.f, 0.f, 0.f}, d[3] = {0.f, 0.f, 0.f};
       int ray_state = 2;
-      if (h == 0) {
+      if (own) {
         if (r >= 0) {
           ray_state = a.state[r];
           for (int c = 0; c < 3; ++c) {
@@ -287,69 +315,71 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) trace_march_kernel(
         // layer 0 of level 0 (the A operand is free: the last GEMM that read
         // it has been drained)
 #pragma unroll 1
-        for (int c = 0; c < NC; ++c)
+        for (int c = grp; c < NC; c += kGroups) {
           bf16::layer0_unit<T, false, U>(sA, w0s, WP, m, c * kKC + h * U, 0, 0.f, x, y, z);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(afull);
+          hand_chunk(c);
+        }
         for (int lev = 0; lev < L; ++lev) {
           const float* wout = wouts + lev * WP;
           const bool next = lev + 1 < L;  // layer 0 of the next level in the last drain
           const float* w0n = w0s + (lev + 1) * 4 * WP;
           float part = 0.f;
           for (int l = 1; l <= nh; ++l, ++k) {
-            if (!fail && !bf16::warp_wait(dfull, (uint32_t)(k & 1), a.status, abort_flag))
+            if (!fail &&
+                !bf16::warp_wait(&dfull[k & 1u], (k >> 1) & 1u, a.status, abort_flag))
               fail = true;
             tc::fence_after_sync();
-            if (!fail) {
+            const uint32_t acc = tl + (k & 1u) * WP;
+            if (fail) {
+            } else if (l < nh) {
 #pragma unroll 1
-              for (int c0 = 0; c0 < NC; c0 += 2) {
-                uint32_t r2[2][U];
-                tc::ld_32x32b<U>(tl + (uint32_t)(c0 * kKC + h * U), r2[0]);
-                if (c0 + 1 < NC) tc::ld_32x32b<U>(tl + (uint32_t)((c0 + 1) * kKC + h * U), r2[1]);
+              for (int c = grp; c < NC; c += kGroups) {
+                const int j0 = c * kKC + h * U;
+                uint32_t rr[U];
+                tc::ld_32x32b<U>(acc + (uint32_t)j0, rr);
                 tc::wait_ld();
+                float v[U];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                  const int c = c0 + u;
-                  if (c >= NC) break;
-                  const int j0 = c * kKC + h * U;
-                  if (l < nh) {
-                    float v[U];
+                for (int jj = 0; jj < U; ++jj) v[jj] = bf16::sin_fast(__uint_as_float(rr[jj]));
+                bf16::store_a_unit<T, U>(sA, m, j0, v);
+                hand_chunk(c);
+              }
+            } else {
+#pragma unroll 1
+              for (int c = 0; c < NC; ++c) {
+                const int j0 = c * kKC + h * U;
+                if (sums) {
+                  uint32_t rr[U];
+                  tc::ld_32x32b<U>(acc + (uint32_t)j0, rr);
+                  tc::wait_ld();
+                  const float4* wo4 = reinterpret_cast<const float4*>(wout + j0);
 #pragma unroll
-                    for (int jj = 0; jj < U; ++jj) v[jj] = bf16::sin_fast(__uint_as_float(r2[u][jj]));
-                    bf16::store_a_unit<T, U>(sA, m, j0, v);
-                  } else {
-                    const float4* wo4 = reinterpret_cast<const float4*>(wout + j0);
+                  for (int j4 = 0; j4 < U / 4; ++j4) {
+                    const float4 wv = wo4[j4];
+                    const float wa[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
-                    for (int j4 = 0; j4 < U / 4; ++j4) {
-                      const float4 wv = wo4[j4];
-                      const float wa[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-                      for (int i = 0; i < 4; ++i)
-                        part = __fmaf_rn(bf16::sin_fast(__uint_as_float(r2[u][4 * j4 + i])), wa[i],
-                                         part);
-                    }
-                    if (next) bf16::layer0_unit<T, false, U>(sA, w0n, WP, m, j0, 0, 0.f, x, y, z);
+                    for (int i = 0; i < 4; ++i)
+                      part = __fmaf_rn(bf16::sin_fast(__uint_as_float(rr[4 * j4 + i])), wa[i],
+                                       part);
                   }
+                }
+                if (firsts && next) {
+                  bf16::layer0_unit<T, false, U>(sA, w0n, WP, m, j0, 0, 0.f, x, y, z);
+                  hand_chunk(c);
                 }
               }
             }
-            const bool hand_over = l < nh || next;  // this drain wrote the next A operand
-            if (hand_over) fence_proxy_async_smem();
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-              if (hand_over) mbar_arrive(afull);
-              mbar_arrive(dempty);
-            }
+            if (lane == 0) mbar_arrive(&dempty[k & 1u]);
           }
-          red[(lev * Q + h) * kM + m] = part;
+          if (sums) red[(lev * Q + h) * kM + m] = part;
         }
         // every level's partial sums written: the h = 0 warps combine the
         // feature splits, gate the levels by band and take the marching step
         fail = bf16::epi_any(fail, kEpiThreads);
         if (fail) break;
-        if (h == 0) {
+        if (own) {
           float sacc = 0.f;
           bool gate = alive;
           for (int lev = 0; lev < L; ++lev) {
@@ -387,7 +417,7 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) trace_march_kernel(
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (warp == kMmaWarp) tc::tmem_dealloc(tmem, WP);
+  if (warp == kMmaWarp) tc::tmem_dealloc(tmem, 2 * WP);
 }
 
 template <int WP, int U, typename T>
@@ -401,7 +431,7 @@ int launch_u(const Args& a, cudaStream_t s) {
   const int64_t sms = sm_count();
   grid = grid < sms ? grid : sms;
   if (grid <= 0) return MPL_OK;
-  trace_march_kernel<WP, U, T><<<(unsigned)grid, bf16::Epi<U>::kThreads, smem, s>>>(a);
+  trace_march_kernel<WP, U, T><<<(unsigned)grid, Roles<U>::kThreads, smem, s>>>(a);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
 }
