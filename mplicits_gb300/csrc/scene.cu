@@ -72,8 +72,9 @@ constexpr int kScanItems = 4;
 constexpr int kScanBlock = kThreads * kScanItems;
 // calc_deltas: triangles a vertex keeps between iterations
 constexpr int kList = 16;
-// resident blocks per SM of its search kernels
-constexpr int kSearchBlocks = 4;
+// resident blocks per SM of its search kernels (four spill: 48.3 against 45.3 ms
+// on the sphere mesh)
+constexpr int kSearchBlocks = 3;
 // warps that share a heavy search, and the listed vertices up to which they
 // take every search (the others would leave warps idle)
 constexpr int kHeavyWarps = 4;
@@ -624,8 +625,8 @@ __global__ void distance_kernel(View S, const float* __restrict__ pts, int64_t n
 // vertex (q, and with it every later decision, stays what it is).
 // Bound: gathers of grid entries that hit L2, in the searches.  On the
 // 523,266-vertex sphere mesh (99 iterations) a search per vertex and step took
-// 204.7 ms (51.8 M searches); with certified stretches 48 ms (1.5 M searches,
-// 26 ms of them in the three steps where most vertices' stretches end at once).
+// 204.7 ms (51.8 M searches); with certified stretches 38 ms (about 2 M
+// searches).
 struct Bisect {
   const float* __restrict__ v;
   int64_t M;
@@ -734,7 +735,7 @@ struct Search {
   float clear;            // listed keys lie below it, no other key does
 };
 
-constexpr int kUnroll = 4;                // entries a thread tests at a time
+constexpr int kUnroll = 2;                // entries a thread tests at a time
 constexpr int kQueue = 32 * (kUnroll + 1);  // per warp: a batch and what they add
 // shared memory of a search by kWarps warps
 template <int kWarps>
@@ -1175,10 +1176,13 @@ __global__ void __launch_bounds__(kWarps > 1 ? kWarps * 32 : kThreads,
     int flags = __float_as_int(st.w);
     uint2 wit = B.wit[i];
     bool shrink;
-    // the stretch to certify: to four times delta (at least eight steps), no
-    // farther than a delta known to be close or the end of the loop
+    // the stretch to certify: half as far again as delta (at least eight
+    // steps; a far ball costs more entries than the searches it saves: to four
+    // times delta 45.3 ms on the sphere mesh, twice 38.2, half again 38.5, a
+    // quarter 41.0), no farther than a delta known to be close or the end of
+    // the loop
     float delta_t = delta + ((flags & kShort) ? 4.f * fabsf(st.x)
-                                              : fmaxf(3.f * delta, 8.f * fabsf(st.x)));
+                                              : fmaxf(0.5f * delta, 8.f * fabsf(st.x)));
     delta_t = fminf(delta_t, B.max_delta + 2.f * fabsf(st.x));
     delta_t = fmaxf(fminf(delta_t, st.z), delta * 1.00001f);
     const V3 qt = ray_point(B, i, delta_t, n);
