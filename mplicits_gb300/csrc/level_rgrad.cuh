@@ -70,7 +70,7 @@ struct Cfg {
   static constexpr uint32_t oWout = oW0 + WP * 16;               // float [WP]
   static constexpr uint32_t oRed = oWout + WP * 4;               // float [Q-1][4][128]
   static constexpr uint32_t oBar = oRed + (Q > 1 ? Q - 1 : 1) * 4 * kM * 4;
-  static constexpr uint32_t kNumBars = 2 * STAGES + bf16::kMaxNC + 1 + 1 + 2 + 1 + 1;
+  static constexpr uint32_t kNumBars = 2 * STAGES + bf16::kMaxNC + 1 + 2 + 2 + 1 + 1;
   static constexpr uint32_t oMisc = oBar + kNumBars * 8;
   static constexpr uint32_t oAx = (oMisc + 16 + 1023) & ~1023u;  // ones tile
   static constexpr uint32_t oBx = oAx + kM * 16 * 2;             // [nh] bias tiles
@@ -104,8 +104,10 @@ __global__ void __launch_bounds__(Roles<U>::kThreads, 1) level_rgrad_kernel(cons
   uint64_t* wempty = bars + S;        // [S]  MMA -> TMA
   uint64_t* achunk = bars + 2 * S;    // [NC] chunk of a forward GEMM's A written (count 4 Q)
   uint64_t* afull = achunk + bf16::kMaxNC;  // a backward GEMM's A written, accumulators read
-  uint64_t* dfull = afull + 1;        // GEMM done
-  uint64_t* redfull = dfull + 1;      // h > 0 partials written (count 4 (Q-1))
+  // [2] GEMM done, in turn: group 0 may still wait for a tile's last GEMM when
+  // the next tile's first one is done
+  uint64_t* dfull = afull + 1;
+  uint64_t* redfull = dfull + 2;      // h > 0 partials written (count 4 (Q-1))
   uint64_t* redfree = redfull + 1;    // h = 0 has read them (count 4)
   uint64_t* gread = redfree + 1;      // B_1's accumulator read (count 4 Q)
   uint64_t* finalb = gread + 1;       // last MMA commit
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(Roles<U>::kThreads, 1) level_rgrad_kernel(cons
     for (int c = 0; c < bf16::kMaxNC; ++c) mbar_init(&achunk[c], 4 * Q);
     mbar_init(afull, kEpiWarps);
     mbar_init(gread, 4 * Q);
-    mbar_init(dfull, 1);
+    for (int b = 0; b < 2; ++b) mbar_init(&dfull[b], 1);
     mbar_init(redfull, 4 * (Q - 1));
     mbar_init(redfree, 4);
     mbar_init(finalb, 1);
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(Roles<U>::kThreads, 1) level_rgrad_kernel(cons
             if (++ws == S) ws = 0, wpar ^= 1u;
           }
           if (!ok) break;
-          tc::commit(dfull);
+          tc::commit(&dfull[(nf + nb) & 1]);
           if (fwd)
             ++nf;
           else
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(Roles<U>::kThreads, 1) level_rgrad_kernel(cons
       float xn = 0.f, yn = 0.f, zn = 0.f;
       float fpart = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
       for (int g = 0; g < G2; ++g, ++k) {
-        if (!bf16::warp_wait(dfull, (uint32_t)(k & 1), a.status, abort_flag)) {
+        if (!bf16::warp_wait(&dfull[k & 1], (uint32_t)((k >> 1) & 1), a.status, abort_flag)) {
           ok = false;
           break;
         }
