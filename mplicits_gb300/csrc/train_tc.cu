@@ -113,6 +113,42 @@ __device__ __forceinline__ void store_unit(uint8_t* sA, __nv_bfloat16* g, int64_
   }
 }
 
+constexpr float kHalfPi = 1.57079632679489662f;
+
+// dz of four features for the four lanes of a point (lane ch of it: value row 0,
+// tangents 1..3), from the value row's phases zv, the lane's own row z (its
+// tangent of z) and ds:
+//   dz_t = cos(zv) ds_t,  dz_v = cos(zv) ds_v - sin(zv) sum_t ds_t z_t.
+// Sine and cosine of a feature are the same for the four lanes, and the sine
+// unit takes 8 cycles a warp and scheduler: lane i takes feature i's two (two
+// sines a lane instead of eight), and the sum over the tangents, which only
+// feature i's lane needs, is a reduce-scatter (three shuffles instead of
+// eight).  The roundings are those of each lane working for itself.
+__device__ __forceinline__ void adjoint4(int ch, int vlane, const float (&zv)[4],
+                                         const float (&z)[4], const float (&ds)[4],
+                                         float (&dz)[4]) {
+  const float lo = (ch & 1) ? zv[1] : zv[0], hi = (ch & 1) ? zv[3] : zv[2];
+  const float mine = (ch & 2) ? hi : lo;
+  float p[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) p[i] = ch ? __fmul_rn(ds[i], z[i]) : 0.f;
+  const float a0 = (ch & 1) ? p[1] : p[0], b0 = (ch & 1) ? p[0] : p[1];
+  const float a1 = (ch & 1) ? p[3] : p[2], b1 = (ch & 1) ? p[2] : p[3];
+  const float r0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, b0, 1));
+  const float r1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, b1, 1));
+  const float keep = (ch & 2) ? r1 : r0, send = (ch & 2) ? r0 : r1;
+  const float tt = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, 2));
+  const float cv = bf16::sin_fast(mine, kHalfPi);
+  const float st = __fmul_rn(bf16::sin_fast(mine), tt);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float c = __shfl_sync(0xffffffffu, cv, vlane + i);
+    const float u = __shfl_sync(0xffffffffu, st, vlane + i);
+    const float t = __fmul_rn(c, ds[i]);
+    dz[i] = ch ? t : __fsub_rn(t, u);
+  }
+}
+
 template <int WP, int STAGES, int U>
 __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) train_tc_kernel(const Args a) {
   using C = Cfg<WP, STAGES, U>;
@@ -128,7 +164,6 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) train_tc_kernel(con
   constexpr int NC = C::NC;
   constexpr int S = STAGES;
   constexpr uint32_t IDESC = tc::idesc_f16kind_f32(kM, WP, Op::kFormat);
-  constexpr float kHalfPi = 1.57079632679489662f;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sA = smem + C::oA;
   uint8_t* sW = smem + C::oW;
@@ -439,17 +474,17 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) train_tc_kernel(con
           tc::wait_ld();
           float v[U];
 #pragma unroll
-          for (int jj = 0; jj < U; ++jj) {
-            const float zo = __uint_as_float(zr[jj]);
-            const float zv = __shfl_sync(0xffffffffu, zo, vlane);
-            const float ds = l < nh ? __uint_as_float(dr[jj]) : __fmul_rn(seed, wout[j0 + jj]);
-            float tt = ch ? __fmul_rn(ds, zo) : 0.f;
-            tt = __fadd_rn(tt, __shfl_xor_sync(0xffffffffu, tt, 1));
-            tt = __fadd_rn(tt, __shfl_xor_sync(0xffffffffu, tt, 2));
-            const float cv = bf16::sin_fast(zv, kHalfPi);
-            const float sv = bf16::sin_fast(zv);
-            const float dz = ch ? __fmul_rn(cv, ds) : __fsub_rn(__fmul_rn(cv, ds), __fmul_rn(sv, tt));
-            v[jj] = valid ? dz : 0.f;
+          for (int j4 = 0; j4 < U; j4 += 4) {
+            float zo[4], zv[4], ds[4], dz[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              zo[i] = __uint_as_float(zr[j4 + i]);
+              zv[i] = __shfl_sync(0xffffffffu, zo[i], vlane);
+              ds[i] = l < nh ? __uint_as_float(dr[j4 + i]) : __fmul_rn(seed, wout[j0 + j4 + i]);
+            }
+            adjoint4(ch, vlane, zv, zo, ds, dz);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[j4 + i] = valid ? dz[i] : 0.f;
           }
           store_unit<U>(sA, dg, grow, m, j0, WP, v);
           fence_proxy_async_smem();
@@ -489,21 +524,15 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) train_tc_kernel(con
               const float ax[4] = {wx.x, wx.y, wx.z, wx.w};
               const float ay[4] = {wy.x, wy.y, wy.z, wy.w};
               const float az[4] = {wz.x, wz.y, wz.z, wz.w};
+              float zt[4], ds[4], dz[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                const int jj = 4 * j4 + i;
-                const float zv = zq[i];
-                const float zt = ch == 1 ? ax[i] : (ch == 2 ? ay[i] : az[i]);
-                const float ds = __uint_as_float(dr[jj]);
-                float tt = ch ? __fmul_rn(ds, zt) : 0.f;
-                tt = __fadd_rn(tt, __shfl_xor_sync(0xffffffffu, tt, 1));
-                tt = __fadd_rn(tt, __shfl_xor_sync(0xffffffffu, tt, 2));
-                const float cv = bf16::sin_fast(zv, kHalfPi);
-                const float sv = bf16::sin_fast(zv);
-                const float dz =
-                    ch ? __fmul_rn(cv, ds) : __fsub_rn(__fmul_rn(cv, ds), __fmul_rn(sv, tt));
-                v[jj] = valid ? dz : 0.f;
+                zt[i] = ch == 1 ? ax[i] : (ch == 2 ? ay[i] : az[i]);
+                ds[i] = __uint_as_float(dr[4 * j4 + i]);
               }
+              adjoint4(ch, vlane, zq, zt, ds, dz);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) v[4 * j4 + i] = valid ? dz[i] : 0.f;
             }
             store_unit<U>(nullptr, dg, grow, m, j0, WP, v);
           }
