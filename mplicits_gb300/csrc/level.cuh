@@ -109,6 +109,24 @@ __device__ __forceinline__ void store_and_band(const LevelArgs& a, bool valid, i
 }
 
 int launch_level_fp32(const LevelArgs& a, cudaStream_t s);
+// Whether the FP32 gradient and backward kernels run n points in half tiles
+// (16 points, two CTAs per SM) instead of full ones (32 points, one CTA): not
+// for the smaller width, whose half tiles lose 5-8% everywhere.  In units of a
+// full tile's time a wave of pairs measured 1.02-1.06, a half tile with an SM
+// to itself 0.61, and a last wave that fills at most half of the SMs 0.4-0.5
+// (it starts while the slower half of each pair still runs; beyond that, two
+// of its tiles can meet on one SM).  Gradient of n points, 256 wide, full and
+// half: 500 99.6 / 60.5 us, 4864 100 / 106, 6000 197 / 149, 7000 197 / 206,
+// 12,000 295 / 307, 30,000 683 / 657.
+inline bool half_tiles(int64_t n, int WP) {
+  if (WP < 128) return false;
+  const int64_t sms = sm_count(), full = (n + 31) / 32, half = (n + 15) / 16;
+  if (half <= sms) return true;
+  const int64_t rest = half % (2 * sms);
+  const double t = 1.05 * (double)(half / (2 * sms)) +
+                   (rest == 0 ? 0.0 : (2 * rest <= sms ? 0.5 : 1.05));
+  return t < (double)((full + sms - 1) / sms);
+}
 int launch_level_split(const LevelArgs& a, cudaStream_t s);
 int launch_level_bf16(const LevelArgs& a, cudaStream_t s);
 int launch_level_f16(const LevelArgs& a, cudaStream_t s);

@@ -22,21 +22,20 @@ namespace mpl {
 
 namespace {
 
-constexpr int kTile = 128;  // points per tile
-constexpr int kKC = 32;     // K rows per weight chunk
-
-// Thread layout of a width: TX threads along the features (8 features each,
-// two float4 groups 4*TX apart) x 16 along the rows (8 rows each: 4 + 4, 64
-// apart), 2*WP threads in all.
-template <int WP>
+// Thread layout of a width and a tile of kTile rows (128, or 64 with two CTAs
+// per SM): TX threads along the features (8 features each, two float4 groups
+// 4*TX apart) x kTile / 8 along the rows (8 rows each: 4 + 4, half a tile
+// apart).
+template <int WP, int kTile>
 struct Fp32Threads {
   static constexpr int TX = WP / 8;
-  static constexpr int kThreads = TX * 16;
+  static constexpr int kThreads = TX * (kTile / 8);
+  static constexpr int kKC = kTile == 128 ? 32 : 16;  // K rows per weight chunk
 };
 
-template <int WP>
+template <int WP, int kTile>
 struct Fp32Smem {
-  static constexpr int FPT = 8;  // features per thread
+  static constexpr int kKC = Fp32Threads<WP, kTile>::kKC;
   static constexpr size_t act = (size_t)WP * kTile * 4;
   static constexpr size_t wbuf = 2ull * kKC * WP * 4;
   static size_t bytes(int nh) {
@@ -45,25 +44,27 @@ struct Fp32Smem {
   }
 };
 
-template <int WP, bool GRAD>
-__global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kernel(const LevelArgs a) {
+template <int WP, bool GRAD, int kTile>
+__global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128 ? 1 : 2)
+    level_fp32_kernel(const LevelArgs a) {
+  constexpr int kKC = Fp32Threads<WP, kTile>::kKC;
   constexpr int PT = GRAD ? kTile / 4 : kTile;  // points per tile
-  constexpr int TX = Fp32Threads<WP>::TX;
-  constexpr int kThreads = Fp32Threads<WP>::kThreads;
+  constexpr int TX = Fp32Threads<WP, kTile>::TX;
+  constexpr int kThreads = Fp32Threads<WP, kTile>::kThreads;
   constexpr int FPT = 8;
   constexpr int NQ = FPT / 4;  // float4 groups of features per thread
   constexpr int CPL = WP / kKC;  // chunks per hidden layer
   extern __shared__ __align__(128) unsigned char smem[];
-  float* act = reinterpret_cast<float*>(smem);                  // [WP][128]
+  float* act = reinterpret_cast<float*>(smem);                  // [WP][kTile]
   float* wbuf = act + WP * kTile;                                // [2][KC][WP]
   float* w0t = wbuf + 2 * kKC * WP;                              // [3][WP]
   float* b0 = w0t + 3 * WP;                                      // [WP]
   const int nh = a.lay.nh;
   float* bh = b0 + WP;                                           // [nh][WP]
   float* wout = bh + (nh > 0 ? nh : 1) * WP;                     // [WP]
-  float* pts = wout + WP;                                        // [128][3]
-  int64_t* pidx = reinterpret_cast<int64_t*>(pts + kTile * 3);   // [128]
-  float* fout = reinterpret_cast<float*>(pidx + kTile);          // [128]
+  float* pts = wout + WP;                                        // [kTile][3]
+  int64_t* pidx = reinterpret_cast<int64_t*>(pts + kTile * 3);   // [kTile]
+  float* fout = reinterpret_cast<float*>(pidx + kTile);          // [kTile]
   uint64_t* bar = reinterpret_cast<uint64_t*>(fout + kTile);     // [2]
 
   const int tid = threadIdx.x;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
     // ---- layer 0: acc = W0 x (+ b0 in the epilogue)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int row = (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
+      const int row = (i < 4) ? ty * 4 + i : kTile / 2 + ty * 4 + (i - 4);
       const int pt = GRAD ? row >> 2 : row;
       const int ch = GRAD ? (i & 3) : 0;  // 0: value row, 1..3: d/dx_(ch-1)
       const float x = pts[pt * 3 + 0], y = pts[pt * 3 + 1], z = pts[pt * 3 + 2];
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
 #pragma unroll 4
           for (int kk = 0; kk < kKC; ++kk) {
             const float4 a0 = act4[(k0 + kk) * (kTile / 4) + ty];
-            const float4 a1 = act4[(k0 + kk) * (kTile / 4) + 16 + ty];
+            const float4 a1 = act4[(k0 + kk) * (kTile / 4) + kTile / 8 + ty];
             const uint64_t av[8] = {bf16::f2pack(a0.x, a0.x), bf16::f2pack(a0.y, a0.y),
                                     bf16::f2pack(a0.z, a0.z), bf16::f2pack(a0.w, a0.w),
                                     bf16::f2pack(a1.x, a1.x), bf16::f2pack(a1.y, a1.y),
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
         // training: keep the pre-activations of every row for the backward
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int row = (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
+          const int row = (i < 4) ? ty * 4 + i : kTile / 2 + ty * 4 + (i - 4);
           const int64_t qq = t * PT + (row >> 2);
           if (qq < n) {
             float* dst = a.pre + (((int64_t)layer * n + qq) * 4 + (i & 3)) * WP;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
             for (int i = 0; i < 8; ++i) s[i] = sinf(__fmul_rn(om, __fadd_rn(acc[i][f], bj)));
           }
           actw[j * (kTile / 4) + ty] = make_float4(s[0], s[1], s[2], s[3]);
-          actw[j * (kTile / 4) + 16 + ty] = make_float4(s[4], s[5], s[6], s[7]);
+          actw[j * (kTile / 4) + kTile / 8 + ty] = make_float4(s[4], s[5], s[6], s[7]);
         }
         __syncthreads();
       } else {
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
         if (tx == 0) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const int row = (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
+            const int row = (i < 4) ? ty * 4 + i : kTile / 2 + ty * 4 + (i - 4);
             const bool value_row = !GRAD || (i & 3) == 0;
             fout[row] = value_row ? __fadd_rn(part[i], bout) : part[i];
           }
@@ -297,18 +298,19 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
     if (!ok) break;
 
     // ---- store / accumulate + fused band compaction
-    if (tid < PT) {
+    if (tid < (PT < 32 ? 32 : PT)) {  // whole warps: the band's ballot
       const int64_t q = t * PT + tid;
       if (GRAD) {
-        const int64_t p = pidx[tid];
-        if (q < n && a.G) {
+        const bool in = tid < PT && q < n;
+        const int64_t p = in ? pidx[tid] : 0;
+        if (in && a.G) {
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
             const float gk = fout[4 * tid + 1 + k];
             a.G[3 * p + k] = a.store_mode == MPL_ACCUMULATE ? __fadd_rn(a.G[3 * p + k], gk) : gk;
           }
         }
-        store_and_band(a, q < n, p, fout[4 * tid]);
+        store_and_band(a, in, p, in ? fout[4 * tid] : 0.f);
       } else {
         store_and_band(a, q < n, pidx[tid], fout[tid]);
       }
@@ -321,21 +323,31 @@ __global__ void __launch_bounds__(Fp32Threads<WP>::kThreads, 1) level_fp32_kerne
   }
 }
 
-template <int WP, bool GRAD>
-int launch_fp32_wp(const LevelArgs& a, cudaStream_t s) {
+template <int WP, bool GRAD, int kTile>
+int launch_fp32_tile(const LevelArgs& a, cudaStream_t s) {
   constexpr int PT = GRAD ? kTile / 4 : kTile;
-  const size_t smem = Fp32Smem<WP>::bytes(a.lay.nh);
-  MPL_CUDA_TRY(cudaFuncSetAttribute(level_fp32_kernel<WP, GRAD>,
+  const size_t smem = Fp32Smem<WP, kTile>::bytes(a.lay.nh);
+  MPL_CUDA_TRY(cudaFuncSetAttribute(level_fp32_kernel<WP, GRAD, kTile>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int64_t grid = sm_count();
+  int64_t grid = (int64_t)sm_count() * (128 / kTile);
   if (!a.n_dev) {
     const int64_t ntiles = (a.n + PT - 1) / PT;
     grid = ntiles < grid ? ntiles : grid;
   }
   if (grid <= 0) return MPL_OK;
-  level_fp32_kernel<WP, GRAD><<<(unsigned)grid, Fp32Threads<WP>::kThreads, smem, s>>>(a);
+  level_fp32_kernel<WP, GRAD, kTile>
+      <<<(unsigned)grid, Fp32Threads<WP, kTile>::kThreads, smem, s>>>(a);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
+}
+
+template <int WP, bool GRAD>
+int launch_fp32_wp(const LevelArgs& a, cudaStream_t s) {
+  if constexpr (GRAD && WP >= 128) {
+    // a device-side count may be anything up to n: full tiles
+    if (!a.n_dev && half_tiles(a.n, WP)) return launch_fp32_tile<WP, GRAD, 64>(a, s);
+  }
+  return launch_fp32_tile<WP, GRAD, 128>(a, s);
 }
 
 template <bool GRAD>

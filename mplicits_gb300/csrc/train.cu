@@ -26,9 +26,6 @@ namespace mpl {
 
 namespace {
 
-constexpr int kRows = 128;  // rows per tile = 32 points x 4
-constexpr int kPts = 32;
-constexpr int kKC = 32;
 
 struct TrainArgs {
   const char* packed;
@@ -51,10 +48,14 @@ struct WgradOut {
 // A thread holds 8 rows x 8 features (two groups of four, 4 TX apart), as in
 // the forward kernel; with 16 features a thread, half the warps, the tile's
 // latencies stood open (15,000 points of a 256-wide level 450 -> 429 us).
-template <int WP>
-__global__ void __launch_bounds__(2 * WP, 1) train_backward_kernel(const TrainArgs a) {
+// kRows rows per tile (128, or 64 with two CTAs per SM): kRows / 4 points x 4.
+template <int WP, int kRows>
+__global__ void __launch_bounds__(WP / 8 * (kRows / 8), kRows == 128 ? 1 : 2)
+    train_backward_kernel(const TrainArgs a) {
+  constexpr int kPts = kRows / 4;
+  constexpr int kKC = kRows == 128 ? 32 : 16;
   constexpr int TX = WP / 8;
-  constexpr int kThreads = 16 * TX;
+  constexpr int kThreads = TX * (kRows / 8);
   constexpr int FPT = 8;
   constexpr int NQ = FPT / 4;
   constexpr int CPL = WP / kKC;
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(2 * WP, 1) train_backward_kernel(const TrainAr
     // d_out of the last hidden layer: seed of the row times W_L
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int row = (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
+      const int row = (i < 4) ? ty * 4 + i : kRows / 2 + ty * 4 + (i - 4);
       const int64_t q = t * kPts + (row >> 2);
       const float sd = q < a.n ? a.seed[q * 4 + (i & 3)] : 0.f;
 #pragma unroll
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(2 * WP, 1) train_backward_kernel(const TrainAr
       // d_a from d_out and this layer's pre-activations
 #pragma unroll
       for (int gq = 0; gq < 2; ++gq) {
-        const int row0 = gq == 0 ? ty * 4 : 64 + ty * 4;
+        const int row0 = gq == 0 ? ty * 4 : kRows / 2 + ty * 4;
         const int64_t q = t * kPts + (row0 >> 2);
         const bool valid = q < a.n;
         const float* pr = a.pre + (((int64_t)l * a.n + q) * 4) * WP;
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(2 * WP, 1) train_backward_kernel(const TrainAr
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
               const int jj = j + r;
-              actw[jj * (kRows / 4) + (gq == 0 ? ty : 16 + ty)] =
+              actw[jj * (kRows / 4) + (gq == 0 ? ty : kRows / 8 + ty)] =
                   make_float4(reinterpret_cast<float*>(&dv[0])[r], reinterpret_cast<float*>(&dv[1])[r],
                               reinterpret_cast<float*>(&dv[2])[r], reinterpret_cast<float*>(&dv[3])[r]);
             }
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(2 * WP, 1) train_backward_kernel(const TrainAr
 #pragma unroll 4
         for (int kk = 0; kk < kKC; ++kk) {
           const float4 a0 = act4[(k0 + kk) * (kRows / 4) + ty];
-          const float4 a1 = act4[(k0 + kk) * (kRows / 4) + 16 + ty];
+          const float4 a1 = act4[(k0 + kk) * (kRows / 4) + kRows / 8 + ty];
           const uint64_t av[8] = {bf16::f2pack(a0.x, a0.x), bf16::f2pack(a0.y, a0.y),
                                   bf16::f2pack(a0.z, a0.z), bf16::f2pack(a0.w, a0.w),
                                   bf16::f2pack(a1.x, a1.x), bf16::f2pack(a1.y, a1.y),
@@ -520,17 +521,27 @@ __global__ void train_batch_kernel(const float* __restrict__ V, int64_t M, int C
   }
 }
 
-template <int WP>
-int launch_backward_wp(const TrainArgs& t, cudaStream_t s) {
+template <int WP, int kRows>
+int launch_backward_rows(const TrainArgs& t, cudaStream_t s) {
+  constexpr int kPts = kRows / 4;
+  constexpr int kKC = kRows == 128 ? 32 : 16;
   const size_t smem = (size_t)WP * kRows * 4 + 2ull * kKC * WP * 4 + WP * 4 + 16;
-  MPL_CUDA_TRY(cudaFuncSetAttribute(train_backward_kernel<WP>,
+  MPL_CUDA_TRY(cudaFuncSetAttribute(train_backward_kernel<WP, kRows>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int64_t grid = sm_count();
+  int64_t grid = (int64_t)sm_count() * (128 / kRows);
   const int64_t ntiles = (t.n + kPts - 1) / kPts;
   grid = ntiles < grid ? ntiles : grid;
-  train_backward_kernel<WP><<<(unsigned)grid, 2 * WP, smem, s>>>(t);
+  train_backward_kernel<WP, kRows><<<(unsigned)grid, WP / 8 * (kRows / 8), smem, s>>>(t);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
+}
+
+template <int WP>
+int launch_backward_wp(const TrainArgs& t, cudaStream_t s) {
+  if constexpr (WP >= 128) {
+    if (half_tiles(t.n, WP)) return launch_backward_rows<WP, 64>(t, s);
+  }
+  return launch_backward_rows<WP, 128>(t, s);
 }
 
 }  // namespace
