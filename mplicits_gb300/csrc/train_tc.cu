@@ -17,8 +17,9 @@
 //    weight-gradient GEMM.
 // 2. train_tc_wgrad_kernel: dW_l = omega_l * sum_rows dz_l (x) s_(l-1), a
 //    GEMM over rows (K = rows) on tcgen05 with both operands MN-major, split
-//    over row blocks, partial sums added atomically.
-// 3. train_tc_ends_kernel: biases, layer 0 and the output layer (SIMT).
+//    over row blocks, partial sums added atomically; and the bias gradients
+//    db_l of the same layers, from the blocks already in shared memory.
+// 3. train_tc_ends_kernel: layer 0 and the output layer (SIMT).
 //
 // With z = omega (W s + b) the pre-activation (omega folded), value row
 // s = sin z_v, tangent rows s = cos(z_v) zt.  Backward, given ds:
@@ -567,15 +568,31 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) train_tc_kernel(con
 // Weight gradients of the hidden layers: for job l, dW_l[j][k] +=
 // omega_l * sum_rows dz_l[row][j] * s_(l-1)[row][k].  M = j (one or two
 // 128-row halves, one TMEM accumulator each), N = k, K = rows in 64-row
-// blocks.  Warps 0-3 read the accumulators out, warp 4 issues the MMAs,
-// warp 5 the bulk copies.
+// blocks.  Warp 4 issues the MMAs, warp 5 the bulk copies; warps 0-3 add up the
+// value rows of each dz block (db_l[j] += omega_l * sum dz_l[value row][j]) and
+// read the accumulators out at the end.
+// Bound: DRAM (6.8 TB/s; each tile is read once).  The bias sums cost it
+// nothing; made by the end-layer kernel, they had it fetch the dz tiles of every
+// layer a second time (1.6 instead of 0.8 GB), and a step of 196,608 points,
+// 256 wide, took 2097 us instead of 1937.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void add8(float (&acc)[8], const uint4& v) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    acc[2 * i] += f.x;
+    acc[2 * i + 1] += f.y;
+  }
+}
+
 constexpr int kWgStages = 3;
 
 struct WgArgs {
   const __nv_bfloat16* A[MPL_MAX_LAYERS];  // dz_l tiles per job
   const __nv_bfloat16* B[MPL_MAX_LAYERS];  // s_(l-1) tiles per job
   float* dW[MPL_MAX_LAYERS];
+  float* db[MPL_MAX_LAYERS];
   float omega[MPL_MAX_LAYERS];
   int64_t nblocks;  // 64-row blocks
   int* status;
@@ -605,7 +622,7 @@ __global__ void __launch_bounds__(192, 1) train_tc_wgrad_kernel(const WgArgs w) 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kWgStages; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], 1 + 4);  // the MMA's commit and the summing warps
     }
     mbar_init(done, 1);
     *abort_flag = 0;
@@ -665,8 +682,54 @@ __global__ void __launch_bounds__(192, 1) train_tc_wgrad_kernel(const WgArgs w) 
       tc::commit(done);
     }
   } else {
+    // bias sums: kSub threads per 8 features; thread `sub` takes the value rows
+    // (every fourth) of its half of every kSub/2-th group of 8 rows, so that a
+    // warp's 16-byte reads use both bank groups that hold value rows.  Sums of
+    // 16 blocks are closed before they join the total.
+    constexpr int kSub = 128 / (WP / 8);
+    const int oct = threadIdx.x / kSub, sub = threadIdx.x % kSub;
+    float tot[8] = {}, run[8] = {};
+    bool ok = true;
+    int64_t i = 0;
+    for (int64_t b = b0; b < b1; ++b, ++i) {
+      const int s = (int)(i % kWgStages);
+      if (!bf16::warp_wait(&full[s], (uint32_t)((i / kWgStages) & 1), w.status, abort_flag)) {
+        ok = false;
+        break;
+      }
+      const uint8_t* o = smem + s * kStage + oct * 1024 + (sub >> 1) * 128 + (sub & 1) * 64;
+      float v[8] = {};
+#pragma unroll
+      for (int k = 0; k < 16 / kSub; ++k)
+        add8(v, *reinterpret_cast<const uint4*>(o + k * (kSub / 2) * 128));
+      // orders these reads before the bulk copy that refills the stage: without
+      // it, sums of 128-wide levels now and then held values of a later block
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+      const bool close = (i & 15) == 15;
+#pragma unroll
+      for (int f = 0; f < 8; ++f) {
+        run[f] += v[f];
+        if (close) {
+          tot[f] += run[f];
+          run[f] = 0.f;
+        }
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < 8; ++f) {
+      tot[f] += run[f];
+#pragma unroll
+      for (int d = kSub / 2; d >= 1; d >>= 1) tot[f] += __shfl_xor_sync(0xffffffffu, tot[f], d);
+    }
+    if (ok && sub == 0) {
+#pragma unroll
+      for (int f = 0; f < 8; ++f)
+        atomicAdd(&w.db[job][oct * 8 + f], __fmul_rn(w.omega[job], tot[f]));
+    }
     // read-out: warp q owns TMEM lanes 32q..32q+31, i.e. j = 128 hh + 32 q + lane
-    const bool ok = bf16::warp_wait(done, 0u, w.status, abort_flag);
+    ok = ok && bf16::warp_wait(done, 0u, w.status, abort_flag);
     if (ok) {
       tc::fence_after_sync();
       float* dW = w.dW[job];
@@ -697,114 +760,90 @@ __global__ void __launch_bounds__(192, 1) train_tc_wgrad_kernel(const WgArgs w) 
 }
 
 // ---------------------------------------------------------------------------
-// Biases, layer 0 and the output layer from the tiles:
-//   db_l[j]  += omega_l * sum_points dz_l[value row][j]        (l = 0..nh)
+// Layer 0 and the output layer from the tiles:
+//   db_0[j]  += omega_0 * sum_points dz_0[value row][j]
 //   dW0[j][c] += omega_0 * sum_points (dz_0[v][j] x_c + dz_0[t_c][j])
 //   dWL[j]   += sum_rows seed_row * s_nh[row][j],  dbL += sum_points seed_v.
-// Block (f8, split): features 8 f8 .. 8 f8 + 7.  Each warp walks 64-row
-// blocks, lane l taking rows l and l + 32, so a warp reads 512 contiguous
-// bytes per operand (one 8-feature column of a block is 1 KiB contiguous).
-// Lanes keep their partial sums across blocks; one warp reduction and one
-// atomic per value at the end.
+// Block (f8, split): features 8 f8 .. 8 f8 + 7.  Each warp walks 32 points at a
+// time, a lane one point: its four rows are 64 contiguous bytes per operand, so
+// the sums need no branch on the row's kind.  Lanes keep their partial sums, two
+// features per instruction, across blocks; one warp reduction and one atomic
+// per value at the end.
 // ---------------------------------------------------------------------------
 struct EndsArgs {
-  const __nv_bfloat16* dz;  // layer 0 of the dz tiles; layer l at + l * lstride
+  const __nv_bfloat16* dz;  // layer 0 of the dz tiles
   const __nv_bfloat16* s_last;
   const float* seeds;
   const float* xyz;
-  int64_t n, nblocks, lstride;
-  int WP, nh;
-  float omega[MPL_MAX_LAYERS];
+  int64_t n;
+  int WP;
+  float omega0;
   float* dW0;
-  float* db[MPL_MAX_LAYERS];
+  float* db0;
   float* dWL;
   float* dbL;
 };
 
-__device__ __forceinline__ void add8(float (&acc)[8], const uint4& v) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    acc[2 * i] += f.x;
-    acc[2 * i + 1] += f.y;
-  }
-}
-
-__device__ __forceinline__ void fma8(float (&acc)[8], const uint4& v, float s) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    acc[2 * i] = __fmaf_rn(s, f.x, acc[2 * i]);
-    acc[2 * i + 1] = __fmaf_rn(s, f.y, acc[2 * i + 1]);
-  }
-}
-
 constexpr int kEndsWarps = 8;
-constexpr int kEndsQ = 3 + 3 + 1;  // db_0..db_2, dW0 x/y/z, dWL
+constexpr int kEndsQ = 1 + 3 + 1;  // db_0, dW0 x/y/z, dWL
+
+// eight BF16 values as four pairs of FP32
+__device__ __forceinline__ void pairs8(uint64_t (&f)[4], const uint4& v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    f[i] = bf16::f2pack(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+}
 
 __global__ void __launch_bounds__(kEndsWarps * 32, 2) train_tc_ends_kernel(const EndsArgs e) {
   __shared__ float part[kEndsWarps][kEndsQ * 8 + 1];
-  const int WP = e.WP, nh = e.nh;
+  const int WP = e.WP;
   const int f8 = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float acc[kEndsQ][8];
+  uint64_t acc2[kEndsQ][4] = {};
   float dbl = 0.f;
+  const uint64_t one = bf16::f2pack(1.f, 1.f);
+  const int64_t stride = (int64_t)gridDim.y * kEndsWarps * 32;
+  for (int64_t p = ((int64_t)blockIdx.y * kEndsWarps + warp) * 32 + lane; p < e.n; p += stride) {
+    const int64_t off = wg_offset(4 * p, f8 * 8, WP);
+    uint4 dv[4], sv[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      dv[c] = *reinterpret_cast<const uint4*>(e.dz + off + 8 * c);
+      sv[c] = *reinterpret_cast<const uint4*>(e.s_last + off + 8 * c);
+    }
+    const float4 sd = *reinterpret_cast<const float4*>(e.seeds + 4 * p);
+    const float xyz[3] = {e.xyz[3 * p], e.xyz[3 * p + 1], e.xyz[3 * p + 2]};
+    const float seed[4] = {sd.x, sd.y, sd.z, sd.w};
+    dbl += sd.x;
+    uint64_t f[4];
+    pairs8(f, dv[0]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc2[0][i] = bf16::ffma2(one, f[i], acc2[0][i]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        acc2[1 + c][i] = bf16::ffma2(bf16::f2pack(xyz[c], xyz[c]), f[i], acc2[1 + c][i]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      pairs8(f, dv[1 + c]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc2[1 + c][i] = bf16::ffma2(one, f[i], acc2[1 + c][i]);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      pairs8(f, sv[c]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        acc2[4][i] = bf16::ffma2(bf16::f2pack(seed[c], seed[c]), f[i], acc2[4][i]);
+    }
+  }
+  float acc[kEndsQ][8];
 #pragma unroll
   for (int qq = 0; qq < kEndsQ; ++qq)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[qq][i] = 0.f;
-  // one 64-row block per iteration, two rows per lane: every load of an
-  // iteration is issued before the arithmetic that uses it, and two CTAs
-  // fit on an SM (128 registers a thread)
-  const int64_t stride = (int64_t)gridDim.y * kEndsWarps;
-  for (int64_t b0 = (int64_t)blockIdx.y * kEndsWarps + warp; b0 < e.nblocks; b0 += stride) {
-    uint4 sv[2], dv[2], d1[2], d2[2];
-    float sd[2], cx[2], cy[2], cz[2];
-    int64_t rowv[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int64_t b = b0 + (u >> 1) * stride;
-      const int64_t row = b * 64 + lane + 32 * (u & 1);
-      rowv[u] = (b < e.nblocks && (row >> 2) < e.n) ? row : -1;
-      if (rowv[u] < 0) continue;
-      const int64_t p = row >> 2;
-      const int ch = (int)(row & 3);
-      const int64_t off = wg_offset(row, f8 * 8, WP);
-      sd[u] = e.seeds[4 * p + ch];
-      sv[u] = *reinterpret_cast<const uint4*>(e.s_last + off);
-      dv[u] = *reinterpret_cast<const uint4*>(e.dz + off);
-      if (ch == 0) {
-        d1[u] = *reinterpret_cast<const uint4*>(e.dz + e.lstride + off);
-        if (nh > 1) d2[u] = *reinterpret_cast<const uint4*>(e.dz + 2 * e.lstride + off);
-        cx[u] = e.xyz[3 * p + 0];
-        cy[u] = e.xyz[3 * p + 1];
-        cz[u] = e.xyz[3 * p + 2];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (rowv[u] < 0) continue;
-      const int ch = (int)(rowv[u] & 3);
-      fma8(acc[6], sv[u], sd[u]);
-      if (ch == 0) {
-        dbl += sd[u];
-        add8(acc[0], dv[u]);
-        fma8(acc[3], dv[u], cx[u]);
-        fma8(acc[4], dv[u], cy[u]);
-        fma8(acc[5], dv[u], cz[u]);
-        add8(acc[1], d1[u]);
-        if (nh > 1) add8(acc[2], d2[u]);
-      } else if (ch == 1) {
-        add8(acc[3], dv[u]);
-      } else if (ch == 2) {
-        add8(acc[4], dv[u]);
-      } else {
-        add8(acc[5], dv[u]);
-      }
-    }
-  }
+    for (int i = 0; i < 4; ++i) bf16::f2unpack(acc2[qq][i], acc[qq][2 * i], acc[qq][2 * i + 1]);
 #pragma unroll
   for (int qq = 0; qq < kEndsQ; ++qq)
 #pragma unroll
@@ -825,10 +864,10 @@ __global__ void __launch_bounds__(kEndsWarps * 32, 2) train_tc_ends_kernel(const
       continue;
     }
     const int qq = t >> 3, j = f8 * 8 + (t & 7);
-    if (qq <= 2) {
-      if (qq <= nh) atomicAdd(&e.db[qq][j], __fmul_rn(e.omega[qq], v));
-    } else if (qq <= 5) {
-      atomicAdd(&e.dW0[j * 3 + (qq - 3)], __fmul_rn(e.omega[0], v));
+    if (qq == 0) {
+      atomicAdd(&e.db0[j], __fmul_rn(e.omega0, v));
+    } else if (qq <= 3) {
+      atomicAdd(&e.dW0[j * 3 + (qq - 1)], __fmul_rn(e.omega0, v));
     } else {
       atomicAdd(&e.dWL[j], v);
     }
@@ -962,6 +1001,7 @@ extern "C" int mpl_train_tc_step(const MplNet* net, const void* packed, const fl
     w.A[l - 1] = a.dz_tiles + (int64_t)l * lstride;
     w.B[l - 1] = a.s_tiles + (int64_t)(l - 1) * lstride;
     w.dW[l - 1] = dW[l];
+    w.db[l - 1] = db[l];
     w.omega[l - 1] = net->omega[l];
   }
   w.nblocks = rows_pad / 64;
@@ -973,7 +1013,7 @@ extern "C" int mpl_train_tc_step(const MplNet* net, const void* packed, const fl
   MPL_CUDA_TRY(cudaStreamWaitEvent(side->s, side->fork, 0));
   st = WP == 256 ? launch_wgrad<256>(w, nh, s) : launch_wgrad<128>(w, nh, s);
   if (st != MPL_OK) return st;
-  // biases, layer 0, output layer
+  // layer 0 and the output layer
   EndsArgs e;
   memset(&e, 0, sizeof(e));
   e.dz = a.dz_tiles;
@@ -981,19 +1021,14 @@ extern "C" int mpl_train_tc_step(const MplNet* net, const void* packed, const fl
   e.seeds = seeds;
   e.xyz = xyz;
   e.n = n;
-  e.nblocks = rows_pad / 64;
-  e.lstride = lstride;
   e.WP = WP;
-  e.nh = nh;
-  for (int l = 0; l <= nh; ++l) {
-    e.omega[l] = net->omega[l];
-    e.db[l] = db[l];
-  }
+  e.omega0 = net->omega[0];
+  e.db0 = db[0];
   e.dW0 = dW[0];
   e.dWL = dW[L - 1];
   e.dbL = db[L - 1];
   int64_t splits = (4 * (int64_t)sm_count()) / (WP / 8);
-  const int64_t wmax = (e.nblocks + kEndsWarps - 1) / kEndsWarps;
+  const int64_t wmax = (n + 32 * kEndsWarps - 1) / (32 * kEndsWarps);
   if (splits > wmax) splits = wmax;
   if (splits < 1) splits = 1;
   train_tc_ends_kernel<<<dim3((unsigned)(WP / 8), (unsigned)splits), kEndsWarps * 32, 0,
