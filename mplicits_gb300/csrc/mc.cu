@@ -3,9 +3,9 @@
 // and the 512 MiB device->host copy before it (i3d/meshing.py:242).
 //
 // The volume is C-order [N][N][N]; a *row* is the N points (i, j, 0..N-1).
-//   count:  one warp per row classifies its points (crossing edges owned by
-//           each point) and cells (case -> triangle count) and writes the
-//           row totals;
+//   count:  one warp per four rows classifies their points (crossing edges
+//           owned by each point) and cells (case -> triangle count) and writes
+//           the row totals;
 //   scan:   exclusive prefix sums of the row totals (int64);
 //   emit:   one CTA per non-empty row rebuilds the in-row vertex prefixes of
 //           the four rows a cell touches with warp scans, writes the row's
@@ -65,86 +65,130 @@ __host__ inline int64_t mc_work_bytes(int64_t N) {
   return align256(R * 4) * 2 + align256(R * 8) * 2 + align256(2 * mc_nblk(N) * 8) + 256;
 }
 
-// Four consecutive values of a row line starting at k (a multiple of 4):
-// one 16-byte load when the grid size is a multiple of 4 (every line then
-// starts 16-byte aligned), otherwise scalar loads; entries past N are 0.
-__device__ __forceinline__ void load4(const float* __restrict__ line, int64_t k, int64_t N,
-                                      bool vec, float (&v)[4]) {
-  if (vec && k + 3 < N) {
-    const float4 f = *reinterpret_cast<const float4*>(line + k);
-    v[0] = f.x;
-    v[1] = f.y;
-    v[2] = f.z;
-    v[3] = f.w;
+// Sign bits (S < iso) of the four values of a line at k (a multiple of 4), bits
+// 0..3: one 16-byte load when the grid size is a multiple of 4 (kVec: every
+// line then starts 16-byte aligned and ends at a multiple of 4), otherwise
+// scalar loads; 0 past N.  Indices are 32-bit (N <= 1024): in 64 bits their
+// arithmetic bounded the counting kernel.
+template <bool kVec>
+__device__ __forceinline__ uint32_t sign4(const float* __restrict__ line, int k, int N,
+                                          float iso) {
+  uint32_t b = 0;
+  if (kVec) {
+    if (k < N) {
+      const float4 f = *reinterpret_cast<const float4*>(line + k);
+      b = (f.x < iso ? 1u : 0u) | (f.y < iso ? 2u : 0u) | (f.z < iso ? 4u : 0u) |
+          (f.w < iso ? 8u : 0u);
+    }
   } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = k + e < N ? line[k + e] : 0.f;
+    for (int e = 0; e < 4; ++e) b |= (k + e < N && line[k + e] < iso ? 1u : 0u) << e;
   }
+  return b;
 }
 
-// Sign bits (S < iso) of the four values of a lane (bits 0..3) and of the
-// value that follows them (bit 4, a separate load that hits the same or the
-// next cache line).
-__device__ __forceinline__ uint32_t sign5(const float* __restrict__ line, int64_t k, int64_t N,
-                                          bool vec, float iso) {
-  float v[4];
-  load4(line, k, N, vec, v);
-  const float nx = k + 4 < N ? line[k + 4] : 0.f;
-  uint32_t b = 0;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) b |= (v[e] < iso ? 1u : 0u) << e;
-  return b | ((k + 4 < N && nx < iso) ? 16u : 0u);
+// Sign of the value after a warp's 128 (lane 31's fifth bit; 0 past the line).
+__device__ __forceinline__ uint32_t sign_after(const float* __restrict__ line, int k, int N,
+                                               float iso, int lane) {
+  return lane == 31 && k + 4 < N && line[k + 4] < iso ? 1u : 0u;
 }
 
-// One warp per row (i, j), 128 points per step (4 per lane): crossing edges
-// owned by each point (along i, j, k, in that order of the mask bits) and the
-// triangle count of each cell (i, j, k) -> (i+1, j+1, k+1).
-__global__ void mc_count_kernel(const float* __restrict__ S, int64_t N, float iso, McWork w) {
+// Bits e of a lane with k + e < N, e = 0..4.
+__device__ __forceinline__ uint32_t in_line5(int k, int N) {
+  const int left = N - k;
+  return left >= 5 ? 31u : (left <= 0 ? 0u : (1u << left) - 1u);
+}
+
+// One warp per strip of kCountRows rows (i, j..), 128 points per step (4 per
+// lane): crossing edges owned by each point (along i, j, k, in that order of
+// the mask bits) and the triangle count of each cell (i, j, k) -> (i+1, j+1,
+// k+1).
+// Bound: L2 and issue.  A strip reads each of its 2 x 5 lines once (a warp per
+// row reads every line four times), all of a step's loads are issued before
+// the first is used, the fifth sign of a lane comes from its neighbour, and
+// the case look-ups are left out where a lane's cells have one sign: with the
+// scans, 512 -> 191 us at 512^3 (eight rows 197), 75 -> 41 us at 256^3.
+constexpr int kCountRows = 4;
+
+template <bool kVec>
+__global__ void __launch_bounds__(256) mc_count_kernel(const float* __restrict__ S, int N,
+                                                       float iso, McWork w) {
+  constexpr int kLines = kCountRows + 1;
   const int lane = threadIdx.x & 31;
-  const int64_t r = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (r >= N * N) return;
-  const int64_t i = r / N, j = r % N;
-  const bool has_i = i + 1 < N, has_j = j + 1 < N;
-  const bool vec = (N & 3) == 0;
-  const float* L00 = S + (i * N + j) * N;
-  const float* L10 = L00 + N * N;
-  const float* L01 = L00 + N;
-  const float* L11 = L10 + N;
-  int nv = 0, nt = 0;
-  for (int64_t k0 = 0; k0 < N; k0 += 128) {
-    const int64_t k = k0 + 4 * lane;
-    const uint32_t a = sign5(L00, k, N, vec, iso);
-    const uint32_t b = has_i ? sign5(L10, k, N, vec, iso) : 0u;
-    const uint32_t c = has_j ? sign5(L01, k, N, vec, iso) : 0u;
-    const uint32_t d = has_i && has_j ? sign5(L11, k, N, vec, iso) : 0u;
+  const int g = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  const int strips = (N + kCountRows - 1) / kCountRows;
+  const int i = g / strips, j0 = (g % strips) * kCountRows;
+  if (i >= N) return;
+  const bool has_i = i + 1 < N;
+  const float* L0 = S + (int64_t)(i * N + j0) * N;
+  uint32_t tot[kCountRows] = {};  // vertices | triangles << 16 (at most 3 N and 5 N)
+  for (int k0 = 0; k0 < N; k0 += 128) {
+    const int k = k0 + 4 * lane;
+    uint32_t a[2][kLines];
+    uint32_t first = 0, after = 0;  // bit 2 q + p: the lines' first and following signs
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (k + e >= N) break;
-      const uint32_t s0 = (a >> e) & 1u;
-      int m = 0;
-      if (has_i && (((b >> e) & 1u) != s0)) m |= 1;
-      if (has_j && (((c >> e) & 1u) != s0)) m |= 2;
-      if (k + e + 1 < N && (((a >> (e + 1)) & 1u) != s0)) m |= 4;
-      nv += __popc(m);
-      if (has_i && has_j && k + e + 1 < N) {
-        // corner q: (i + (q & 1), j + ((q >> 1) & 1), k + e + (q >> 2))
-        const uint32_t cs = ((a >> e) & 1u) | (((b >> e) & 1u) << 1) | (((c >> e) & 1u) << 2) |
-                            (((d >> e) & 1u) << 3) | (((a >> (e + 1)) & 1u) << 4) |
-                            (((b >> (e + 1)) & 1u) << 5) | (((c >> (e + 1)) & 1u) << 6) |
-                            (((d >> (e + 1)) & 1u) << 7);
-        nt += c_tri_count[cs];
+    for (int q = 0; q < kLines; ++q)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const bool in = j0 + q < N && (p == 0 || has_i);
+        const float* line = L0 + p * N * N + q * N;
+        a[p][q] = in ? sign4<kVec>(line, k, N, iso) : 0u;
+        after |= (in ? sign_after(line, k, N, iso, lane) : 0u) << (2 * q + p);
       }
+#pragma unroll
+    for (int q = 0; q < kLines; ++q)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) first |= (a[p][q] & 1u) << (2 * q + p);
+    const uint32_t next = __shfl_down_sync(0xffffffffu, first, 1);
+    if (lane < 31) after = next;
+    const uint32_t in5 = in_line5(k, N);
+#pragma unroll
+    for (int q = 0; q < kLines; ++q)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) a[p][q] |= ((after >> (2 * q + p)) & 1u) << 4;
+#pragma unroll
+    for (int q = 0; q < kCountRows; ++q) {
+      const bool has_j = j0 + q + 1 < N;
+      if (j0 + q >= N) break;
+      const uint32_t s = a[0][q], b = has_i ? a[1][q] : s, c = has_j ? a[0][q + 1] : s;
+      const uint32_t d = has_i && has_j ? a[1][q + 1] : s;
+      if (((s | b | c | d) == 0u) || ((s & b & c & d) == in5)) continue;  // one sign
+      const uint32_t pts = in5 & 15u, cells = in5 >> 1;  // points, points with a successor
+      uint32_t v = __popc((s ^ b) & pts) + __popc((s ^ c) & pts) + __popc((s ^ (s >> 1)) & cells);
+      if (has_i && has_j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (!((cells >> e) & 1u)) continue;
+          // corner: (i + (x & 1), j + ((x >> 1) & 1), k + e + (x >> 2))
+          const uint32_t cs = ((s >> e) & 1u) | (((b >> e) & 1u) << 1) | (((c >> e) & 1u) << 2) |
+                              (((d >> e) & 1u) << 3) | (((s >> (e + 1)) & 1u) << 4) |
+                              (((b >> (e + 1)) & 1u) << 5) | (((c >> (e + 1)) & 1u) << 6) |
+                              (((d >> (e + 1)) & 1u) << 7);
+          v += (uint32_t)c_tri_count[cs] << 16;
+        }
+      }
+      tot[q] += v;
     }
   }
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    nv += __shfl_xor_sync(0xffffffffu, nv, o);
-    nt += __shfl_xor_sync(0xffffffffu, nt, o);
+  for (int q = 0; q < kCountRows; ++q) {
+    const uint32_t t = __reduce_add_sync(0xffffffffu, tot[q]);
+    if (lane == 0 && j0 + q < N) {
+      w.row_v[i * N + j0 + q] = (int32_t)(t & 0xffffu);
+      w.row_t[i * N + j0 + q] = (int32_t)(t >> 16);
+    }
   }
-  if (lane == 0) {
-    w.row_v[r] = nv;
-    w.row_t[r] = nt;
-  }
+}
+
+int launch_count(const float* S, int64_t N, float iso, const McWork& w, cudaStream_t s) {
+  const int64_t warps = N * ((N + kCountRows - 1) / kCountRows);
+  const unsigned grid = (unsigned)((warps + 7) / 8);
+  if ((N & 3) == 0)
+    mc_count_kernel<true><<<grid, 256, 0, s>>>(S, (int)N, iso, w);
+  else
+    mc_count_kernel<false><<<grid, 256, 0, s>>>(S, (int)N, iso, w);
+  MPL_LAUNCH_CHECK();
+  return MPL_OK;
 }
 
 // block-wide exclusive scan of one int64 per thread (blockDim.x a multiple
@@ -246,154 +290,203 @@ __global__ void mc_scan_add(int64_t N, McWork w) {
   w.pre_t[r] += w.blk[2 * b + 1];
 }
 
-__device__ __forceinline__ float grad_axis(const float* __restrict__ S, int64_t N,
-                                           const int64_t idx[3], int axis) {
-  int64_t lo[3] = {idx[0], idx[1], idx[2]};
-  int64_t hi[3] = {idx[0], idx[1], idx[2]};
-  if (idx[axis] > 0) lo[axis] -= 1;
-  if (idx[axis] + 1 < N) hi[axis] += 1;
-  const float d = __fsub_rn(S[(hi[0] * N + hi[1]) * N + hi[2]], S[(lo[0] * N + lo[1]) * N + lo[2]]);
-  return __fdiv_rn(d, (float)(hi[axis] - lo[axis]));
+// Central difference at point p along the axis of the given stride, one-sided at
+// the first and last of the N points (x: the point's index on the axis).
+__device__ __forceinline__ float grad_axis(const float* __restrict__ S, int N, int p, int x,
+                                           int stride) {
+  const int lo = x > 0 ? 1 : 0, hi = x + 1 < N ? 1 : 0;
+  const float d = __fsub_rn(S[p + hi * stride], S[p - lo * stride]);
+  return __fdiv_rn(d, (float)(hi + lo));
 }
 
 constexpr int kEmitThreads = 128;
 constexpr int kMaxN = 1024;
 
+// One warp: the crossing-edge masks (with the point's sign in bit 3) and the
+// in-line vertex prefix of line (ri, rj), kSteps x 128 points at a time, and
+// (list given) the line's vertices as 4 k + axis.  Returns their number.
+template <int kSteps, bool kVec>
+__device__ __forceinline__ int emit_line(const float* __restrict__ S, int N, float iso, int ri,
+                                         int rj, int lane, int16_t* pre, uint8_t* msk,
+                                         uint16_t* list) {
+  const bool has_i = ri + 1 < N, has_j = rj + 1 < N;
+  const float* L = S + (ri * N + rj) * N;
+  int carry = 0;
+  for (int k0 = 0; k0 < N; k0 += 128 * kSteps) {
+    uint32_t a[kSteps], b[kSteps], c[kSteps], after[kSteps];
+#pragma unroll
+    for (int t = 0; t < kSteps; ++t) {
+      const int k = k0 + 128 * t + 4 * lane;
+      a[t] = sign4<kVec>(L, k, N, iso);
+      after[t] = sign_after(L, k, N, iso, lane);
+      b[t] = has_i ? sign4<kVec>(L + N * N, k, N, iso) : a[t];
+      c[t] = has_j ? sign4<kVec>(L + N, k, N, iso) : a[t];
+    }
+    uint64_t x = 0;  // vertices of the lane's points, 16 bits a step (at most 12)
+#pragma unroll
+    for (int t = 0; t < kSteps; ++t) {
+      const int k = k0 + 128 * t + 4 * lane;
+      const uint32_t next = __shfl_down_sync(0xffffffffu, a[t], 1);
+      a[t] |= (lane < 31 ? next & 1u : after[t]) << 4;
+      const uint32_t in5 = in_line5(k, N), pts = in5 & 15u, succ = in5 >> 1;
+      b[t] = (a[t] ^ b[t]) & pts;           // from here on the crossings along i,
+      c[t] = (a[t] ^ c[t]) & pts;           // along j
+      after[t] = (a[t] ^ (a[t] >> 1)) & succ;  // and along k
+      x |= (uint64_t)(__popc(b[t]) + __popc(c[t]) + __popc(after[t])) << (16 * t);
+    }
+    const uint64_t own = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const uint64_t total = __shfl_sync(0xffffffffu, x, 31);
+    x -= own;
+#pragma unroll
+    for (int t = 0; t < kSteps; ++t) {
+      const int k = k0 + 128 * t + 4 * lane;
+      int run = carry + (int)((x >> (16 * t)) & 0xffffu);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (k + e < N) {
+          const uint32_t m = ((b[t] >> e) & 1u) | (((c[t] >> e) & 1u) << 1) |
+                             (((after[t] >> e) & 1u) << 2);
+          pre[k + e] = (int16_t)run;
+          msk[k + e] = (uint8_t)(m | (((a[t] >> e) & 1u) << 3));
+          if (list) {
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax)
+              if ((m >> ax) & 1u) list[run + __popc(m & ((1u << ax) - 1u))] = (uint16_t)(4 * (k + e) + ax);
+          }
+          run += __popc(m);
+        }
+      }
+      carry += (int)((total >> (16 * t)) & 0xffffu);
+    }
+  }
+  return carry;
+}
+
 // One CTA (4 warps) per row r = (i, j); rows without vertices or triangles
 // return at once.
-//   1. warp w walks line (i + (w >> 1), j + (w & 1)), 128 points per step:
-//      the crossing-edge mask and sign bit of each point and its in-line
-//      vertex prefix (warp scan), into shared memory;
-//   2. the vertices of line (i, j) (interpolation, central-difference
-//      normals);
+//   1. warp w walks line (i + (w >> 1), j + (w & 1)), 512 points per step (128
+//      where the line is no longer): the crossing-edge mask and sign bit of
+//      each point and its in-line vertex prefix (warp scan), into shared
+//      memory, and for line (i, j) the list of its vertices;
+//   2. the vertices of line (i, j), one a thread (interpolation,
+//      central-difference normals);
 //   3. the triangles of the cells of row (i, j): each thread takes four
 //      consecutive cells, the cases come from the sign bits of the four
 //      lines, one block scan orders them.
-__global__ void __launch_bounds__(kEmitThreads) mc_emit_kernel(
-    const float* __restrict__ S, int64_t N, float iso, float vs, float o0, float o1, float o2,
+// Bound: latency (a chain of loads, scans and barriers per row, ten CTAs
+// per SM).  The loads of a step are all issued before the first is used, the
+// four scans of a step are one, the vertices come from a list, indices are
+// 32-bit: 1015 -> 593 us at 512^3 (459,208 vertices), 191 -> 130 us at 256^3.
+// Ten CTAs per SM in the launch bounds: 9 646, 11 658, 12 657 us; several rows
+// per CTA are no faster (2: 669, 8: 674 us with 12).
+template <bool kVec>
+__global__ void __launch_bounds__(kEmitThreads, 10) mc_emit_kernel(
+    const float* __restrict__ S, int N, float iso, float vs, float o0, float o1, float o2,
     McWork w, float* __restrict__ verts, float* __restrict__ normals, float* __restrict__ values,
     int32_t* __restrict__ faces, int64_t max_verts, int64_t max_tris) {
   // in-line vertex prefix (< 3 kMaxN) and, per point, the crossing-edge mask
   // (bits 0-2: along i, j, k) with the point's sign S < iso in bit 3
   __shared__ int16_t pre[4][kMaxN];
-  __shared__ uint8_t msk[4][kMaxN];
-  const int64_t r = blockIdx.x;
-  const int64_t i = r / N, j = r % N;
+  __shared__ __align__(4) uint8_t msk[4][kMaxN];
+  __shared__ uint16_t list[3 * kMaxN];  // vertices of line (i, j): 4 k + axis
+  __shared__ int64_t line_v[4];         // first vertex of the four lines
+  __shared__ int line_n;                // vertices of line (i, j)
+  const int r = blockIdx.x;
+  const int i = r / N, j = r % N;
   if (w.row_v[r] == 0 && w.row_t[r] == 0) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const float org[3] = {o0, o1, o2};
 
   // 1. masks, prefixes and signs of the four lines
   {
-    const int64_t ri = i + (wid >> 1), rj = j + (wid & 1);
+    const int ri = i + (wid >> 1), rj = j + (wid & 1);
     if (ri < N && rj < N) {
-      const bool vec = (N & 3) == 0;
-      const bool has_i = ri + 1 < N, has_j = rj + 1 < N;
-      const float* L = S + (ri * N + rj) * N;
-      int32_t carry = 0;
-      for (int64_t k0 = 0; k0 < N; k0 += 128) {
-        const int64_t k = k0 + 4 * lane;
-        const uint32_t a = sign5(L, k, N, vec, iso);
-        const uint32_t b = has_i ? sign5(L + N * N, k, N, vec, iso) : 0u;
-        const uint32_t c = has_j ? sign5(L + N, k, N, vec, iso) : 0u;
-        int m[4], cnt = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t s0 = (a >> e) & 1u;
-          int me = 0;
-          if (k + e < N) {
-            if (has_i && (((b >> e) & 1u) != s0)) me |= 1;
-            if (has_j && (((c >> e) & 1u) != s0)) me |= 2;
-            if (k + e + 1 < N && (((a >> (e + 1)) & 1u) != s0)) me |= 4;
-          }
-          m[e] = me;
-          cnt += __popc(me);
-        }
-        int x = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
-        }
-        int run = carry + x - cnt;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (k + e < N) {
-            pre[wid][k + e] = (int16_t)run;
-            msk[wid][k + e] = (uint8_t)(m[e] | (((a >> e) & 1u) << 3));
-          }
-          run += __popc(m[e]);
-        }
-        carry += __shfl_sync(0xffffffffu, x, 31);
-      }
+      if (lane == 0) line_v[wid] = w.pre_v[ri * N + rj];
+      uint16_t* own = wid == 0 ? list : nullptr;
+      const int cnt = N <= 128
+                          ? emit_line<1, kVec>(S, N, iso, ri, rj, lane, pre[wid], msk[wid], own)
+                          : emit_line<4, kVec>(S, N, iso, ri, rj, lane, pre[wid], msk[wid], own);
+      if (wid == 0 && lane == 0) line_n = cnt;
     }
   }
   __syncthreads();
 
   // 2. vertices of line (i, j)
-  const int64_t vbase = w.pre_v[r];
-  for (int64_t k = threadIdx.x; k < N; k += kEmitThreads) {
-    const int m = msk[0][k] & 7;
-    if (!m) continue;
-    int64_t v = vbase + pre[0][k];
-    const int64_t p = (i * N + j) * N + k;
-    for (int a = 0; a < 3; ++a) {
-      if (!(m & (1 << a))) continue;
-      if (v < max_verts) {
-        const int64_t idx0[3] = {i, j, k};
-        int64_t idx1[3] = {i, j, k};
-        idx1[a] += 1;
-        const float v0 = S[p];
-        const float v1 = S[(idx1[0] * N + idx1[1]) * N + idx1[2]];
-        const float t = __fdiv_rn(__fsub_rn(iso, v0), __fsub_rn(v1, v0));
-        float n[3];
+  const int64_t vbase = line_v[0];
+  const int nv = line_n;
+  for (int q = threadIdx.x; q < nv; q += kEmitThreads) {
+    const int64_t v = vbase + q;
+    if (v >= max_verts) break;
+    const int a = list[q] & 3;
+    const int k = list[q] >> 2;
+    const int idx0[3] = {i, j, k};
+    const int stride[3] = {N * N, N, 1};
+    const int p0 = r * N + k, p1 = p0 + (a == 0 ? N * N : (a == 1 ? N : 1));
+    const float v0 = S[p0], v1 = S[p1];
+    const float t = __fdiv_rn(__fsub_rn(iso, v0), __fsub_rn(v1, v0));
+    float n[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          float c = (float)idx0[d];
-          if (d == a) c = __fadd_rn(c, t);
-          verts[3 * v + d] = __fadd_rn(__fmul_rn(c, vs), org[d]);
-          const float g0 = grad_axis(S, N, idx0, d);
-          const float g1 = grad_axis(S, N, idx1, d);
-          n[d] = __fadd_rn(g0, __fmul_rn(t, __fsub_rn(g1, g0)));
-        }
-        float l2 = __fmul_rn(n[0], n[0]);
-        l2 = __fadd_rn(l2, __fmul_rn(n[1], n[1]));
-        l2 = __fadd_rn(l2, __fmul_rn(n[2], n[2]));
-        const float len = __fsqrt_rn(l2);
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          normals[3 * v + d] = len > 0.0f ? __fdiv_rn(n[d], len) : 0.0f;
-        if (values) values[v] = v0 > v1 ? v0 : v1;
-      }
-      ++v;
+    for (int d = 0; d < 3; ++d) {
+      float c = (float)idx0[d];
+      if (d == a) c = __fadd_rn(c, t);
+      verts[3 * v + d] = __fadd_rn(__fmul_rn(c, vs), org[d]);
+      const float g0 = grad_axis(S, N, p0, idx0[d], stride[d]);
+      const float g1 = grad_axis(S, N, p1, idx0[d] + (d == a), stride[d]);
+      n[d] = __fadd_rn(g0, __fmul_rn(t, __fsub_rn(g1, g0)));
     }
+    float l2 = __fmul_rn(n[0], n[0]);
+    l2 = __fadd_rn(l2, __fmul_rn(n[1], n[1]));
+    l2 = __fadd_rn(l2, __fmul_rn(n[2], n[2]));
+    const float len = __fsqrt_rn(l2);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) normals[3 * v + d] = len > 0.0f ? __fdiv_rn(n[d], len) : 0.0f;
+    if (values) values[v] = v0 > v1 ? v0 : v1;
   }
 
   // 3. triangles of the cells of row (i, j), four consecutive cells a thread
   if (i + 1 >= N || j + 1 >= N) return;
   int64_t tcarry = w.pre_t[r];
-  for (int64_t k0 = 0; k0 < N - 1; k0 += 4 * kEmitThreads) {
-    const int64_t kb = k0 + 4 * threadIdx.x;
-    int cs[4], nts[4], ntot = 0;
+  for (int k0 = 0; k0 < N - 1; k0 += 4 * kEmitThreads) {
+    const int kb = k0 + 4 * threadIdx.x;
+    // signs of the four lines (line (di, dj) = di * 2 + dj) at kb .. kb + 4
+    const uint32_t in5 = in_line5(kb, N);
+    uint32_t sg[4] = {}, any = 0, all = 31;
+    if (kb < N) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int64_t k = kb + e;
-      int c = 0;
-      if (k < N - 1) {
-        // corner q: (i + (q & 1), j + ((q >> 1) & 1), k + (q >> 2)); line (di, dj) = di * 2 + dj
+      for (int l = 0; l < 4; ++l) {
+        const uint32_t x = (*reinterpret_cast<const uint32_t*>(&msk[l][kb]) >> 3) & 0x01010101u;
+        sg[l] = (x | (x >> 7) | (x >> 14) | (x >> 21)) & 15u;
+        if (kb + 4 < N) sg[l] |= ((uint32_t)msk[l][kb + 4] >> 3 & 1u) << 4;
+        sg[l] &= in5;
+        any |= sg[l];
+        all &= sg[l];
+      }
+    }
+    int cs[4] = {}, nts[4] = {}, ntot = 0;
+    if (any && all != in5) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        // corner q: (i + (q & 1), j + ((q >> 1) & 1), k + (q >> 2))
+        if (!((in5 >> (e + 1)) & 1u)) break;
+        int c = 0;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-          c |= (int)((msk[((q & 1) << 1) | ((q >> 1) & 1)][k + (q >> 2)] >> 3) & 1) << q;
+          c |= (int)((sg[((q & 1) << 1) | ((q >> 1) & 1)] >> (e + (q >> 2))) & 1u) << q;
+        cs[e] = c;
+        nts[e] = c_tri_count[c];
+        ntot += nts[e];
       }
-      cs[e] = c;
-      nts[e] = k < N - 1 ? c_tri_count[c] : 0;
-      ntot += nts[e];
     }
     int64_t tot;
     int64_t t = tcarry + block_exclusive_scan(ntot, &tot);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int64_t k = kb + e;
+      const int k = kb + e;
       for (int q = 0; q < nts[e]; ++q, ++t) {
         if (t >= max_tris) break;
 #pragma unroll
@@ -401,9 +494,8 @@ __global__ void __launch_bounds__(kEmitThreads) mc_emit_kernel(
           const int ed = c_tri_edges[cs[e]][3 * q + sidx];
           const int axis = c_edge[ed][0];
           const int row = c_edge[ed][1] * 2 + c_edge[ed][2];
-          const int64_t kk = k + c_edge[ed][3];
-          const int64_t rr = (i + c_edge[ed][1]) * N + (j + c_edge[ed][2]);
-          const int64_t vid = w.pre_v[rr] + pre[row][kk] +
+          const int kk = k + c_edge[ed][3];
+          const int64_t vid = line_v[row] + pre[row][kk] +
                               __popc((int)msk[row][kk] & ((1 << axis) - 1));
           faces[3 * t + sidx] = (int32_t)vid;
         }
@@ -411,6 +503,17 @@ __global__ void __launch_bounds__(kEmitThreads) mc_emit_kernel(
     }
     tcarry += tot;
   }
+}
+
+int launch_emit(const float* S, int64_t N, float iso, float vs, const float* origin,
+                const McWork& w, float* verts, float* normals, float* values, int32_t* faces,
+                int64_t max_verts, int64_t max_tris, cudaStream_t s) {
+  auto* kernel = (N & 3) == 0 ? &mc_emit_kernel<true> : &mc_emit_kernel<false>;
+  kernel<<<(unsigned)(N * N), kEmitThreads, 0, s>>>(S, (int)N, iso, vs, origin[0], origin[1],
+                                                    origin[2], w, verts, normals, values, faces,
+                                                    max_verts, max_tris);
+  MPL_LAUNCH_CHECK();
+  return MPL_OK;
 }
 
 // Per-device one-time set-up (case tables here, the no-allocation
@@ -456,8 +559,8 @@ extern "C" int mpl_mc_count(const float* S, int64_t N, float iso, void* workspac
   cudaStream_t s = (cudaStream_t)stream;
   McWork w = mc_work(workspace, N);
   const int64_t R = N * N;
-  mc_count_kernel<<<(unsigned)((R + 7) / 8), 256, 0, s>>>(S, N, iso, w);
-  MPL_LAUNCH_CHECK();
+  st = launch_count(S, N, iso, w, s);
+  if (st != MPL_OK) return st;
   const int64_t nblk = mc_nblk(N);
   mc_scan_blocks<<<(unsigned)nblk, 256, 0, s>>>(N, w);
   MPL_LAUNCH_CHECK();
@@ -480,11 +583,8 @@ extern "C" int mpl_mc_emit(const float* S, int64_t N, float iso, float voxel_siz
   if (st != MPL_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
   McWork w = mc_work(const_cast<void*>(workspace), N);
-  mc_emit_kernel<<<(unsigned)(N * N), kEmitThreads, 0, s>>>(
-      S, N, iso, voxel_size, origin[0], origin[1], origin[2], w, verts, normals, values, faces,
-      max_verts, max_tris);
-  MPL_LAUNCH_CHECK();
-  return MPL_OK;
+  return launch_emit(S, N, iso, voxel_size, origin, w, verts, normals, values, faces, max_verts,
+                     max_tris, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -559,8 +659,8 @@ extern "C" int mpl_mc_noalloc(const float* S, int64_t N, float iso, float voxel_
   cudaStream_t s = (cudaStream_t)stream;
   McWork w = mc_work(ws, N);
   const int64_t R = N * N;
-  mc_count_kernel<<<(unsigned)((R + 7) / 8), 256, 0, s>>>(S, N, iso, w);
-  MPL_LAUNCH_CHECK();
+  st = launch_count(S, N, iso, w, s);
+  if (st != MPL_OK) return st;
   const int64_t nblk = mc_nblk(N);
   mc_scan_blocks<<<(unsigned)nblk, 256, 0, s>>>(N, w);
   MPL_LAUNCH_CHECK();
@@ -568,9 +668,6 @@ extern "C" int mpl_mc_noalloc(const float* S, int64_t N, float iso, float voxel_
   MPL_LAUNCH_CHECK();
   mc_scan_add<<<(unsigned)((R + 255) / 256), 256, 0, s>>>(N, w);
   MPL_LAUNCH_CHECK();
-  mc_emit_kernel<<<(unsigned)R, kEmitThreads, 0, s>>>(S, N, iso, voxel_size, origin[0],
-                                                       origin[1], origin[2], w, verts, normals,
-                                                       values, faces, max_verts, max_tris);
-  MPL_LAUNCH_CHECK();
-  return MPL_OK;
+  return launch_emit(S, N, iso, voxel_size, origin, w, verts, normals, values, faces, max_verts,
+                     max_tris, s);
 }
