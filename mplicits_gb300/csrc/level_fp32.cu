@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
               }
             }
           }
+          fence_proxy_async_smem();  // these reads before the copy that refills the stage
           __syncthreads();
         }
         if (!ok) break;

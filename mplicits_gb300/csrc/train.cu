@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(WP / 8 * (kRows / 8), kRows == 128 ? 1 : 2)
             }
           }
         }
+        fence_proxy_async_smem();  // these reads before the copy that refills the stage
         __syncthreads();
       }
 #pragma unroll
