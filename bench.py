@@ -9,7 +9,7 @@ gen_mc_coordinate_grid; bands delta0 = 0.05, delta1 = 0.01; marching cubes at
 level 1 on band 1, level 2 on band 2, marching cubes (count + emit) on the
 device.  ``value`` is grid points per second of that step with the 16-bit
 tcgen05 kernels (FP16 operands, the form that meets the SDF error target;
-BF16 beside it); the same step with the plain FP32 kernels, the error of each
+BF16 beside it); the same step with the FP32 kernels, the error of each
 against the FP64 oracle, the end-to-end number through the public API with
 host buffers, the CPU baseline and the roofline of the dominant kernel are in
 the same JSON line, next to the training step, sphere tracing, the batched
@@ -375,7 +375,7 @@ def e2e_run(levels_np, N, device, K, W, precision):
         step()
     torch.cuda.synchronize()
     dt = (time.perf_counter() - t0) / K
-    launches = 3 + 5 + 3 * 4  # levels, MC, re-packing each level's weights
+    launches = 3 + 5 + 3 * 3  # levels, MC, re-packing each level's weights
     return dt, h2d, d2h[0], launches
 
 
@@ -425,7 +425,10 @@ TRAIN_SURFACE = 1 << 16  # surface samples per batch; rows = 3x (surface, offset
 # layers over the four rows
 _FWD_TANGENT = 2 * (3 * 256 + 2 * 256 * 256 + 256) + 3 * 2 * (2 * 256 * 256 + 256)
 TRAIN_FLOP_PER_ROW = 3 * _FWD_TANGENT + 2 * (2 * 4 * 2 * 256 * 256)
-TRAIN_LAUNCHES_PER_STEP = 7  # batch, 2 frozen gradients, fused step, weight GEMM, ends, Adam
+# batch, 2 frozen gradients, fused step, weight GEMM, ends, Adam, 3 of the re-packing
+TRAIN_LAUNCHES_PER_STEP = 7 + 3
+# batch, 2 frozen gradients, forward, loss, backward, 2 weight gradients, Adam, re-packing
+TRAIN_LAUNCHES_PER_STEP_FP32 = 9 + 3
 
 
 def train_surface(n=1 << 18, seed=1):
@@ -471,7 +474,8 @@ def train_bench(levels_np, device, K, W, precision="bf16"):
             "flop_per_row": TRAIN_FLOP_PER_ROW,
             "achieved_tflops": TRAIN_FLOP_PER_ROW * rows / (ms * 1e-3) / 1e12,
             "last_losses": [float(x) for x in losses.cpu()],
-            "gpu_launches": K * (TRAIN_LAUNCHES_PER_STEP if precision == "bf16" else 10)}
+            "gpu_launches": K * (TRAIN_LAUNCHES_PER_STEP if precision == "bf16"
+                                 else TRAIN_LAUNCHES_PER_STEP_FP32)}
 
 
 def train_cpu_baseline(levels_np, rows=3072, steps=3):
@@ -565,7 +569,7 @@ def deltas_bench(device, K, W):
                                       [0.0, 0.1, 0.5, 0.9, 1.0], device=device)).cpu()],
             "e2e": {"value": M / (e2e_ms * 1e-3), "unit": "vertices/s", "ms_per_call": e2e_ms,
                     "h2d_bytes_per_step": V.nbytes, "d2h_bytes_per_step": M * 7 * 4},
-            "gpu_launches": K * (DELTAS_ITERS + 2)}
+            "gpu_launches": K * (3 * DELTAS_ITERS + 2)}
 
 
 def deltas_cpu_baseline(iters, n=16384):

@@ -45,7 +45,8 @@ enum {
 
 /* arithmetic of the hidden-layer GEMMs */
 enum {
-  MPL_FP32 = 0, /* plain form: FP32 SIMT FMAs, accurate sinf               */
+  MPL_FP32 = 0, /* FP32 accuracy: split FP16 operands on tcgen05 for levels
+                   with a hidden GEMM, FP32 FMAs for gradients and the rest */
   MPL_BF16 = 1, /* tcgen05 BF16 MMAs, FP32 accumulate in TMEM, FP32 layer 0 */
   MPL_F16 = 2   /* the same kernels with FP16 operands: same speed, 8x finer
                    rounding of the sine activations (all within [-1, 1])   */
