@@ -109,6 +109,21 @@ __device__ __forceinline__ void store_and_band(const LevelArgs& a, bool valid, i
 }
 
 int launch_level_fp32(const LevelArgs& a, cudaStream_t s);
+// Thread layout of the FP32 kernels' register tiles: TX threads along the
+// features, the rest along the rows, a warp being 8 x 4 of them (lane bits 0, 3
+// and 4 along the features, so that the quarter of a warp that one 16-byte read
+// serves at a time is 2 x 4).  With a row of 32 threads along the features, a
+// warp's reads of a K row took 10 shared-memory cycles, its stores of the next
+// operand 32; gradient of 14,592 points, 256 wide, 295 -> 272 us (lane bits
+// 0, 1, 2 along the features 286, bits 0, 1, 3 275, bits 0, 2, 4 274).
+template <int TX>
+__device__ __forceinline__ void fp32_tile_thread(int tid, int& tx, int& ty) {
+  constexpr int WX = TX / 8;  // warps along the features
+  const int warp = tid >> 5, lane = tid & 31;
+  tx = (warp % WX) * 8 + ((lane & 1) | ((lane >> 2) & 6));
+  ty = (warp / WX) * 4 + ((lane >> 1) & 3);
+}
+
 // Whether the FP32 gradient and backward kernels run n points in half tiles
 // (16 points, two CTAs per SM) instead of full ones (32 points, one CTA): not
 // for the smaller width, whose half tiles lose 5-8% everywhere.  In units of a
@@ -117,7 +132,8 @@ int launch_level_fp32(const LevelArgs& a, cudaStream_t s);
 // (it starts while the slower half of each pair still runs; beyond that, two
 // of its tiles can meet on one SM).  Gradient of n points, 256 wide, full and
 // half: 500 99.6 / 60.5 us, 4864 100 / 106, 6000 197 / 149, 7000 197 / 206,
-// 12,000 295 / 307, 30,000 683 / 657.
+// 12,000 295 / 307, 30,000 683 / 657 (since then both forms are faster: half
+// tiles 500 54.6, 6000 129, 30,000 574 us; full ones 4864 88.7, 7000 175).
 inline bool half_tiles(int64_t n, int WP) {
   if (WP < 128) return false;
   const int64_t sms = sm_count(), full = (n + 31) / 32, half = (n + 15) / 16;

@@ -40,7 +40,7 @@ struct Fp32Smem {
   static constexpr size_t wbuf = 2ull * kKC * WP * 4;
   static size_t bytes(int nh) {
     return act + wbuf + 3 * WP * 4 + WP * 4 + (size_t)(nh > 0 ? nh : 1) * WP * 4 + WP * 4 +
-           kTile * 3 * 4 + kTile * 8 + kTile * 4 + 2 * 8 + 16;
+           kTile * 3 * 4 + kTile * 8 + kTile * 4 * (WP / 64) + 2 * 8 + 16;
   }
 };
 
@@ -64,12 +64,12 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
   float* wout = bh + (nh > 0 ? nh : 1) * WP;                     // [WP]
   float* pts = wout + WP;                                        // [kTile][3]
   int64_t* pidx = reinterpret_cast<int64_t*>(pts + kTile * 3);   // [kTile]
-  float* fout = reinterpret_cast<float*>(pidx + kTile);          // [kTile]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(fout + kTile);     // [2]
+  float* fout = reinterpret_cast<float*>(pidx + kTile);          // [WP / 64][kTile]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(fout + kTile * (WP / 64));  // [2]
 
   const int tid = threadIdx.x;
-  const int tx = tid % TX;
-  const int ty = tid / TX;
+  int tx, ty;
+  fp32_tile_thread<TX>(tid, tx, ty);
   const float4* act4 = reinterpret_cast<const float4*>(act);
 
   const int64_t n = level_point_count(a);
@@ -154,7 +154,9 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
         // ---- hidden GEMM: acc[p][j] = sum_k act[k][p] * Wt[k][j], two
         // features per FMA instruction (the same roundings; the FMA pipe takes
         // as long, but the issue slots it frees go to the shared-memory reads:
-        // gradient of 15,000 points, 256 wide, 454 -> 397 us)
+        // gradient of 15,000 points, 256 wide, 454 -> 397 us).  Sixteen
+        // K rows unrolled keep enough reads in flight: 14,592 points, 4 / 8 / 16
+        // rows 272 / 262 / 260 us, 6000 points in half tiles 140 / 133 / 129 us
         uint64_t acc2[8][FPT / 2];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
           }
           const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(wbuf + (g & 1) * kKC * WP);
           const int k0 = c * kKC;
-#pragma unroll 4
+#pragma unroll 16
           for (int kk = 0; kk < kKC; ++kk) {
             const float4 a0 = act4[(k0 + kk) * (kTile / 4) + ty];
             const float4 a1 = act4[(k0 + kk) * (kTile / 4) + kTile / 8 + ty];
@@ -283,14 +285,13 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
 #pragma unroll
-          for (int o = TX / 2; o >= 1; o >>= 1) part[i] += __shfl_xor_sync(0xffffffffu, part[i], o);
+          for (int o : {16, 8, 1}) part[i] += __shfl_xor_sync(0xffffffffu, part[i], o);  // over tx
         }
-        if (tx == 0) {
+        if ((tx & 7) == 0) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int row = (i < 4) ? ty * 4 + i : kTile / 2 + ty * 4 + (i - 4);
-            const bool value_row = !GRAD || (i & 3) == 0;
-            fout[row] = value_row ? __fadd_rn(part[i], bout) : part[i];
+            fout[(tx >> 3) * kTile + row] = part[i];
           }
         }
         __syncthreads();
@@ -299,6 +300,12 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
     if (!ok) break;
 
     // ---- store / accumulate + fused band compaction
+    auto row_sum = [&](int row) {
+      float s = fout[row];
+#pragma unroll
+      for (int h = 1; h < WP / 64; ++h) s = __fadd_rn(s, fout[h * kTile + row]);
+      return s;
+    };
     if (tid < (PT < 32 ? 32 : PT)) {  // whole warps: the band's ballot
       const int64_t q = t * PT + tid;
       if (GRAD) {
@@ -307,13 +314,13 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
         if (in && a.G) {
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
-            const float gk = fout[4 * tid + 1 + k];
+            const float gk = row_sum(4 * tid + 1 + k);
             a.G[3 * p + k] = a.store_mode == MPL_ACCUMULATE ? __fadd_rn(a.G[3 * p + k], gk) : gk;
           }
         }
-        store_and_band(a, in, p, in ? fout[4 * tid] : 0.f);
+        store_and_band(a, in, p, in ? __fadd_rn(row_sum(4 * tid), bout) : 0.f);
       } else {
-        store_and_band(a, q < n, pidx[tid], fout[tid]);
+        store_and_band(a, q < n, pidx[tid], __fadd_rn(row_sum(tid), bout));
       }
     }
     __syncthreads();
