@@ -63,17 +63,26 @@ class PackedLevel:
 
     def get(self, model):
         lins = model.linears()
-        first = lins[0].weight
-        key = [model.w0, model.ww, first.device]
+        key = [model.w0, model.ww]
+        computed = False
         for lin in lins:
             own = lin._parameters  # a plain lookup where nothing is parametrized
-            for p in (own.get("weight"), own.get("bias")):
+            for name in ("weight", "bias"):
+                p = own.get(name)
                 if p is None:
-                    key += [p.data_ptr() for p in (lin.weight, lin.bias)]
-                    key += [p._version for p in (lin.weight, lin.bias)]
-                    break
-                key.append(p.data_ptr())
-                key.append(p._version)
+                    # a computed weight is another tensor on each access: what it
+                    # is computed from is watched instead (below); a tensor that
+                    # is a plain attribute stays the same one
+                    computed = True
+                    p = lin.__dict__.get(name)
+                if p is not None:
+                    key.append(p.data_ptr())  # of any device: addresses are unified
+                    key.append(p._version)
+        sources = ()
+        if computed:
+            sources = (*model.parameters(), *model.buffers())
+            for p in sources:
+                key += [p.data_ptr(), p._version]
         if key == self.key:
             return self.net, self.buf
         net = model.mpl_net()
@@ -81,17 +90,18 @@ class PackedLevel:
         nbytes = ctypes.c_int64(0)
         capi.check(lib.mpl_net_packed_bytes(ctypes.byref(net), ctypes.byref(nbytes)),
                    "mpl_net_packed_bytes")
-        dev = first.device
+        ws = [l.weight.detach().contiguous().float() for l in lins]
+        bs = [l.bias.detach().contiguous().float() for l in lins]
+        dev = ws[0].device
         buf = torch.empty(nbytes.value + 256, dtype=torch.uint8, device=dev)
         off = (-buf.data_ptr()) % 256
         view = buf[off:off + nbytes.value]
-        ws = [l.weight.detach().contiguous().float() for l in lins]
-        bs = [l.bias.detach().contiguous().float() for l in lins]
         wp = (ctypes.c_void_p * len(ws))(*[w.data_ptr() for w in ws])
         bp = (ctypes.c_void_p * len(bs))(*[b.data_ptr() for b in bs])
         capi.check(lib.mpl_net_pack(ctypes.byref(net), wp, bp, capi.ptr(view),
                                     capi.stream_ptr()), "mpl_net_pack")
-        self._keep = (buf, ws, bs)
+        # the sources too: while they are held, no other tensor has their address
+        self._keep = (buf, ws, bs, [p.detach() for p in sources])
         self.key, self.buf, self.net = key, view, net
         return net, view
 
