@@ -199,7 +199,9 @@ class SIREN(nn.Module):
 
     # -- topology --------------------------------------------------------
     def linears(self):
-        return [blk._modules["0"] for blk in self._modules["net"]._modules.values()]
+        # the first child of each block, whatever it is called (plain lookups:
+        # indexing a Sequential costs a microsecond each)
+        return [next(iter(blk._modules.values())) for blk in self._modules["net"]._modules.values()]
 
     def omegas(self):
         out = []

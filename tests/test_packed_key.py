@@ -122,3 +122,14 @@ def test_repacked_when_changed_and_only_then(lib, make, dtype):
             m.packed()
             m.packed()
             assert lib.packs == i + 2
+
+
+def test_a_layer_of_any_name(lib):
+    """Blocks are indexed, whatever their children are called."""
+    from collections import OrderedDict
+    m = _siren()
+    lin, act = m.net[1][0], m.net[1][1]
+    m.net[1] = torch.nn.Sequential(OrderedDict(linear=lin, act=act))
+    assert m.linears()[1] is lin
+    m.packed()
+    assert lib.packs == 1
