@@ -33,14 +33,18 @@ LOSSES = {"residual": (capi.MPL_LOSS_RESIDUAL, DEFAULT_WEIGHTS),
 
 
 class _Scratch:
-    """Per-model buffers of the backward, grown on demand."""
+    """Per-model buffers of the backward, grown on demand and made anew when the
+    level's layers or device are others."""
 
     def __init__(self, model):
         self.model = model
         self.n = -1
+        self.made_for = None
 
     def ensure(self, n, device):
-        if n <= self.n:
+        lins = self.model.linears()
+        dims = [(l.out_features, l.in_features) for l in lins]
+        if n <= self.n and (dims, device) == self.made_for:
             return
         net = self.model.mpl_net()
         fl = ctypes.c_int64(0)
@@ -52,11 +56,11 @@ class _Scratch:
         self.g = torch.empty(n, 3, dtype=torch.float32, device=device)
         self.seeds = torch.empty(n, 4, dtype=torch.float32, device=device)
         self.n = n
+        self.made_for = (dims, device)
         # padded gradient buffers, one per nn.Linear weight and bias, in one
         # allocation (zeroed and copied by one launch each), every part at a
         # multiple of 256 bytes
         wp = _padded_width(self.model)
-        lins = self.model.linears()
         L = len(lins)
         self.shapes = []
         for l in range(L):
@@ -70,8 +74,8 @@ class _Scratch:
         parts = self.parts(self.flat)
         self.dW, self.db = parts[0::2], parts[1::2]
         # whether the parameters have exactly the padded shapes
-        self.exact = all(tuple(p.shape) == s for l in range(L) for p, s in zip(
-            (lins[l].weight, lins[l].bias), self.shapes[2 * l:2 * l + 2]))
+        self.exact = all(d == s and d[:1] == b for d, s, b in zip(
+            dims, self.shapes[0::2], self.shapes[1::2]))
 
     def parts(self, flat):
         """The views of a flat gradient buffer, weight and bias per layer."""
