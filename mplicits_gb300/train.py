@@ -256,7 +256,6 @@ class ResidualTrainer:
         self.exp_avg_sq = [torch.zeros_like(p) for p in self.params]
         self.t = 0
         self.loss_sums = torch.zeros(4, dtype=torch.float32, device=self.params[0].device)
-        self._scale_n = None  # (n, scale / n) of the last batch size
         self._scale = torch.tensor([w[k] for k in self.names], dtype=torch.float32,
                                    device=self.params[0].device)
 
@@ -267,10 +266,9 @@ class ResidualTrainer:
         return self._loss_and_grads(x, normals, sdf, own=True)
 
     def _terms(self, n):
-        """The weighted loss terms from the sums over n points."""
-        if self._scale_n is None or self._scale_n[0] != n:
-            self._scale_n = (n, self._scale / n)
-        return self.loss_sums[:len(self.names)] * self._scale_n[1]
+        """The weighted loss terms from the sums over n points (scale / n is not
+        kept: made while a CUDA graph is captured, it has no value outside it)."""
+        return self.loss_sums[:len(self.names)] * (self._scale / n)
 
     def _loss_and_grads(self, x, normals, sdf, own):
         x = x.detach().float().reshape(-1, 3).contiguous()
