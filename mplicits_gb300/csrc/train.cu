@@ -344,20 +344,25 @@ int launch_wgrad(const TrainArgs& t, int WP, const WgradOut& out, cudaStream_t s
 
 // Layer 0 (3 inputs): dW0[j][c] += sum_q da_v[j] x_qc + da_tc[j]; db0[j] += da_v[j].
 // Output layer: dWL[j] += sum_rows seed_row out_(L-1)[row][j]; dbL += seed_v.
-// Thread j of a block, four points' loads in flight; each block covers a
-// contiguous point range and adds its partial sums atomically.  dbL, a sum of
-// signed seeds that mostly cancel, is one block's (the last), in double: its
+// Thread j of one of a block's kEndsGroups groups, four points' loads in flight;
+// each group covers a contiguous point range, the groups' sums are added in
+// shared memory and the block's go out atomically.  (A block a group of 16 points
+// is as fast, but its 938 partial sums of 15,000 points, added in a row, made the
+// first layer's gradients 1.4 and the output's 1.5 times as far off.)  dbL, a sum
+// of signed seeds that mostly cancel, is one block's (the last), in double: its
 // float partial sums in atomic order moved it by 1e-6 from run to run.
-// Bound: the latency of the rows' loads (15,000 points 76 -> 59 us).
-__global__ void __launch_bounds__(256) train_wgrad_ends_kernel(const TrainArgs a, int WP,
-                                                               float* dW0, float* db0, float* dWL,
-                                                               float* dbL) {
+// Bound: the latency of the rows' loads.
+constexpr int kEndsGroups = 4;
+
+__global__ void __launch_bounds__(256 * kEndsGroups)
+    train_wgrad_ends_kernel(const TrainArgs a, int WP, float* dW0, float* db0, float* dWL,
+                            float* dbL) {
   const int nh = a.lay.nh;
   if (blockIdx.x == gridDim.x - 1) {
     double b = 0.0;
     for (int64_t q = threadIdx.x; q < a.n; q += blockDim.x) b += (double)a.seed[q * 4];
     for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-    __shared__ double part[8];
+    __shared__ double part[8 * kEndsGroups];
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = b;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -366,36 +371,47 @@ __global__ void __launch_bounds__(256) train_wgrad_ends_kernel(const TrainArgs a
     }
     return;
   }
-  const int64_t nb = gridDim.x - 1;
-  const int64_t per = (a.n + nb - 1) / nb;
-  const int64_t q_begin = blockIdx.x * per;
+  __shared__ float part[kEndsGroups - 1][5][256];
+  const int j = threadIdx.x % WP, grp = threadIdx.x / WP;
+  const int64_t ng = (int64_t)(gridDim.x - 1) * kEndsGroups;
+  const int64_t per = (a.n + ng - 1) / ng;
+  const int64_t q_begin = ((int64_t)blockIdx.x * kEndsGroups + grp) * per;
   const int64_t q_end = q_begin + per < a.n ? q_begin + per : a.n;
   const float om = a.omega[nh];
-  for (int j = threadIdx.x; j < WP; j += blockDim.x) {
-    float w0x = 0.f, w0y = 0.f, w0z = 0.f, b0 = 0.f, wl = 0.f;
+  float w0x = 0.f, w0y = 0.f, w0z = 0.f, b0 = 0.f, wl = 0.f;
 #pragma unroll 4
-    for (int64_t q = q_begin; q < q_end; ++q) {
-      const float* d = a.da + (q * 4) * WP;  // layer 0
-      const float dv = d[j];
-      w0x = __fadd_rn(w0x, __fmaf_rn(dv, a.xyz[3 * q + 0], d[1 * WP + j]));
-      w0y = __fadd_rn(w0y, __fmaf_rn(dv, a.xyz[3 * q + 1], d[2 * WP + j]));
-      w0z = __fadd_rn(w0z, __fmaf_rn(dv, a.xyz[3 * q + 2], d[3 * WP + j]));
-      b0 = __fadd_rn(b0, dv);
-      const float* pr = a.pre + (((int64_t)nh * a.n + q) * 4) * WP;
-      const float4 sd = *reinterpret_cast<const float4*>(a.seed + q * 4);
-      float s, c;
-      sincosf(__fmul_rn(om, pr[j]), &s, &c);
-      const float oc = __fmul_rn(om, c);
-      float t = __fmul_rn(sd.y, pr[1 * WP + j]);
-      t = __fmaf_rn(sd.z, pr[2 * WP + j], t);
-      t = __fmaf_rn(sd.w, pr[3 * WP + j], t);
-      wl = __fmaf_rn(sd.x, s, __fmaf_rn(oc, t, wl));
+  for (int64_t q = q_begin; q < q_end; ++q) {
+    const float* d = a.da + (q * 4) * WP;  // layer 0
+    const float dv = d[j];
+    w0x = __fadd_rn(w0x, __fmaf_rn(dv, a.xyz[3 * q + 0], d[1 * WP + j]));
+    w0y = __fadd_rn(w0y, __fmaf_rn(dv, a.xyz[3 * q + 1], d[2 * WP + j]));
+    w0z = __fadd_rn(w0z, __fmaf_rn(dv, a.xyz[3 * q + 2], d[3 * WP + j]));
+    b0 = __fadd_rn(b0, dv);
+    const float* pr = a.pre + (((int64_t)nh * a.n + q) * 4) * WP;
+    const float4 sd = *reinterpret_cast<const float4*>(a.seed + q * 4);
+    float s, c;
+    sincosf(__fmul_rn(om, pr[j]), &s, &c);
+    const float oc = __fmul_rn(om, c);
+    float t = __fmul_rn(sd.y, pr[1 * WP + j]);
+    t = __fmaf_rn(sd.z, pr[2 * WP + j], t);
+    t = __fmaf_rn(sd.w, pr[3 * WP + j], t);
+    wl = __fmaf_rn(sd.x, s, __fmaf_rn(oc, t, wl));
+  }
+  const float own[5] = {w0x, w0y, w0z, b0, wl};
+  if (grp > 0) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) part[grp - 1][i][j] = own[i];
+  }
+  __syncthreads();
+  if (grp == 0) {
+    float* const dst[5] = {dW0 + j * 3, dW0 + j * 3 + 1, dW0 + j * 3 + 2, db0 + j, dWL + j};
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      float v = own[i];
+#pragma unroll
+      for (int g = 0; g < kEndsGroups - 1; ++g) v = __fadd_rn(v, part[g][i][j]);
+      atomicAdd(dst[i], v);
     }
-    atomicAdd(&dW0[j * 3 + 0], w0x);
-    atomicAdd(&dW0[j * 3 + 1], w0y);
-    atomicAdd(&dW0[j * 3 + 2], w0z);
-    atomicAdd(&db0[j], b0);
-    atomicAdd(&dWL[j], wl);
   }
 }
 
@@ -638,10 +654,12 @@ extern "C" int mpl_train_backward(const MplNet* net, const void* packed, const f
     st = WP == 64 ? launch_wgrad<64>(t, WP, out, s) : launch_wgrad<128>(t, WP, out, s);
     if (st != MPL_OK) return st;
   }
-  // 16 points a block, up to 4096 blocks, and the one of dbL
-  const int64_t eb = (n + 15) / 16 < 4096 ? (n + 15) / 16 : 4096;
-  train_wgrad_ends_kernel<<<(unsigned)(eb + 1), WP < 256 ? WP : 256, 0, s>>>(t, WP, dW[0], db[0],
-                                                                       dW[L - 1], db[L - 1]);
+  // 64 points a block, up to two waves of blocks, and the one of dbL (up to 4096
+  // blocks: 196,608 points 100 us slower at 256 wide, and the first layer's
+  // gradients 1.3 times as far from float64)
+  const int64_t eb = (n + 63) / 64 < 4 * sm_count() ? (n + 63) / 64 : 4 * sm_count();
+  train_wgrad_ends_kernel<<<(unsigned)(eb + 1), WP * kEndsGroups, 0, s>>>(
+      t, WP, dW[0], db[0], dW[L - 1], db[L - 1]);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
 }
