@@ -300,8 +300,9 @@ int mpl_train_loss(int64_t n, const float* f_dev, const float* g_dev, const floa
  * the backward through the level's forward-mode graph (double backward of
  * the input gradient included).  dW[l] / db[l] are device buffers of the
  * padded shapes ([WP][3] for layer 0, [WP][WP] hidden, [WP] output; bias
- * [WP], output bias [1]); the call ADDS into them.  `da` is scratch of the
- * same size as the pre-activations.  Replaces autograd's backward of
+ * [WP], output bias [1]), at any float address (16-byte aligned hidden dW[l]
+ * are added to four values at a time); the call ADDS into them.  `da` is
+ * scratch of the same size as the pre-activations.  Replaces autograd's backward of
  * torch.autograd.grad(..., create_graph=True) in the reference trainers. */
 int mpl_train_backward(const MplNet* net, const void* packed_dev, const float* xyz_dev, int64_t n,
                        const float* pre_dev, const float* seeds_dev, float* da_dev,

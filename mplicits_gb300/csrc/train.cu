@@ -226,7 +226,8 @@ __global__ void __launch_bounds__(WP / 8 * (kRows / 8), kRows == 128 ? 1 : 2)
 // w cos(w a_v) a_t), one sincosf per point and feature.  A CTA holds a T x T
 // tile of dW in registers (T/16 squared per thread) and walks its points four
 // at a time (16 rows), the next ones on their way while the products run;
-// partial sums go out as 16-byte atomic adds.
+// partial sums go out as 16-byte atomic adds (single ones into a buffer that is
+// not 16-byte aligned).
 // Bound: the FP32 FMA pipe.  The split over points fills two CTAs per SM
 // (train_wgrad_blocks): with a fixed 4096 points a CTA, 64 x 64 tiles and a
 // sine per row, 15,000 points of a 256-wide level took 3.25 ms a layer on 64
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
     __syncthreads();
   }
   float* dW = out.dW[l];
+  const bool vec = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;  // the caller's buffer
 #pragma unroll
   for (int u = 0; u < E; ++u) {
     const int j = j0 + (u / 4) * 64 + tj * 4 + (u & 3);
@@ -322,7 +324,15 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
       float4 p;
       bf16::f2unpack(acc[u][v / 2], p.x, p.y);
       bf16::f2unpack(acc[u][v / 2 + 1], p.z, p.w);
-      atomicAdd(reinterpret_cast<float4*>(dW + (int64_t)j * WP + k0 + v * 16 + tk * 4), p);
+      float* d = dW + (int64_t)j * WP + k0 + v * 16 + tk * 4;
+      if (vec) {
+        atomicAdd(reinterpret_cast<float4*>(d), p);
+      } else {
+        atomicAdd(d, p.x);
+        atomicAdd(d + 1, p.y);
+        atomicAdd(d + 2, p.z);
+        atomicAdd(d + 3, p.w);
+      }
     }
   }
   if (k0 == 0 && tid < T) atomicAdd(&out.db[l][j0 + tid], bacc);
