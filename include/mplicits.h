@@ -319,7 +319,7 @@ int mpl_train_tc_scratch_bytes(const MplNet* net, int64_t n, int64_t* bytes);
  * sums into loss_sums[4], seeds [n, 4] written, 16-byte aligned), the
  * backward through the forward-mode graph (double backward included) and
  * every weight gradient, ADDED into the padded buffers dW[l] / db[l] of
- * mpl_train_backward.  Replaces the reference trainers' forward, loss and
+ * mpl_train_backward, the hidden dW[l] 16-byte aligned.  Replaces the reference trainers' forward, loss and
  * loss.backward() (experiment_scripts/train_sdf_on_neighborhood_fine.py:
  * 247-250 with i3d/loss_functions.py:347-394; the coarse trainer with
  * true_sdf).  Levels with 1 or 2 hidden GEMMs of padded width 128 or 256. */

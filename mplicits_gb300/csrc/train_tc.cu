@@ -969,6 +969,8 @@ extern "C" int mpl_train_tc_step(const MplNet* net, const void* packed, const fl
   if (nh < 1 || nh > 2 || (WP != 128 && WP != 256)) return MPL_ERR_UNSUPPORTED;
   for (int l = 0; l < L; ++l)
     if (!dW[l] || !db[l]) return MPL_ERR_INVALID_ARG;
+  for (int l = 1; l <= nh; ++l)  // 16-byte atomics
+    if (n > 0 && ((uintptr_t)dW[l] & 15) != 0) return MPL_ERR_INVALID_ARG;
   int64_t need = 0;
   mpl_train_tc_scratch_bytes(net, n, &need);
   if (scratch_bytes < need) return MPL_ERR_CAPACITY;
