@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(WP / 8 * (kRows / 8), kRows == 128 ? 1 : 2)
   constexpr int NQ = FPT / 4;
   constexpr int CPL = WP / kKC;
   extern __shared__ __align__(128) unsigned char smem[];
-  float* act = reinterpret_cast<float*>(smem);  // d_a, [WP][128] feature-major
+  float* act = reinterpret_cast<float*>(smem);  // d_a, [WP][kRows] feature-major
   float* wbuf = act + WP * kRows;                // [2][KC][WP]
   float* wout = wbuf + 2 * kKC * WP;             // [WP]
   uint64_t* bar = reinterpret_cast<uint64_t*>(wout + WP);
@@ -226,13 +226,13 @@ __global__ void __launch_bounds__(WP / 8 * (kRows / 8), kRows == 128 ? 1 : 2)
 // w cos(w a_v) a_t), one sincosf per point and feature.  A CTA holds a T x T
 // tile of dW in registers (T/16 squared per thread) and walks its points four
 // at a time (16 rows), the next ones on their way while the products run;
-// partial sums go out as 16-byte atomic adds (single ones into a buffer that is
-// not 16-byte aligned).
+// partial sums go out as 16-byte atomic adds (kVec), or as single ones where a
+// caller's buffer is not 16-byte aligned.
 // Bound: the FP32 FMA pipe.  The split over points fills two CTAs per SM
 // (train_wgrad_blocks): with a fixed 4096 points a CTA, 64 x 64 tiles and a
 // sine per row, 15,000 points of a 256-wide level took 3.25 ms a layer on 64
 // CTAs; now 0.16 ms on 304.
-template <int T>
+template <int T, bool kVec>
 __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainArgs a, int WP,
                                                                     WgradOut out) {
   constexpr int E = T / 16;            // values of each axis per thread
@@ -315,7 +315,6 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
     __syncthreads();
   }
   float* dW = out.dW[l];
-  const bool vec = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;  // the caller's buffer
 #pragma unroll
   for (int u = 0; u < E; ++u) {
     const int j = j0 + (u / 4) * 64 + tj * 4 + (u & 3);
@@ -325,7 +324,7 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
       bf16::f2unpack(acc[u][v / 2], p.x, p.y);
       bf16::f2unpack(acc[u][v / 2 + 1], p.z, p.w);
       float* d = dW + (int64_t)j * WP + k0 + v * 16 + tk * 4;
-      if (vec) {
+      if (kVec) {
         atomicAdd(reinterpret_cast<float4*>(d), p);
       } else {
         atomicAdd(d, p.x);
@@ -346,8 +345,10 @@ int launch_wgrad(const TrainArgs& t, int WP, const WgradOut& out, cudaStream_t s
   int64_t splits = (2 * (int64_t)sm_count() + all - 1) / all;
   const int64_t most = (t.n + 63) / 64;
   splits = splits < most ? splits : most;
-  train_wgrad_hidden_kernel<T>
-      <<<dim3((unsigned)splits, (unsigned)all), 256, 0, s>>>(t, WP, out);
+  bool vec = true;
+  for (int l = 1; l <= t.lay.nh; ++l) vec = vec && ((uintptr_t)out.dW[l] & 15) == 0;
+  auto* kernel = vec ? &train_wgrad_hidden_kernel<T, true> : &train_wgrad_hidden_kernel<T, false>;
+  kernel<<<dim3((unsigned)splits, (unsigned)all), 256, 0, s>>>(t, WP, out);
   MPL_LAUNCH_CHECK();
   return MPL_OK;
 }
