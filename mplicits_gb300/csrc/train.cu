@@ -229,9 +229,9 @@ __global__ void __launch_bounds__(WP / 8 * (kRows / 8), kRows == 128 ? 1 : 2)
 // partial sums go out as 16-byte atomic adds (kVec), or as single ones where a
 // caller's buffer is not 16-byte aligned.
 // Bound: the FP32 FMA pipe.  The split over points fills two CTAs per SM
-// (train_wgrad_blocks): with a fixed 4096 points a CTA, 64 x 64 tiles and a
-// sine per row, 15,000 points of a 256-wide level took 3.25 ms a layer on 64
-// CTAs; now 0.16 ms on 304.
+// (launch_wgrad): with a fixed 4096 points a CTA, 64 x 64 tiles and a sine per
+// row, 15,000 points of a 256-wide level took 3.25 ms a layer on 64 CTAs; now
+// 0.16 ms on 304.
 template <int T, bool kVec>
 __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainArgs a, int WP,
                                                                     WgradOut out) {
@@ -338,11 +338,15 @@ __global__ void __launch_bounds__(256, 2) train_wgrad_hidden_kernel(const TrainA
 }
 
 // Blocks that share the points of one tile: two per SM over all tiles, of 64
-// points at least (less would be mostly the atomic adds of the tile).
+// points at least (less would be mostly the atomic adds of the tile).  So many
+// waves of them that a block, a serial FP32 sum, has 4096 points at most whatever
+// the batch: 5174 in one wave, 196,608 points 256 wide, gave gradients 1.1 times as
+// far from float64.  (48 blocks of 4096, 1.3 waves, take 9.3 ms instead of 8.6.)
 template <int T>
 int launch_wgrad(const TrainArgs& t, int WP, const WgradOut& out, cudaStream_t s) {
   const int per_layer = (WP / T) * (WP / T), all = per_layer * t.lay.nh;
   int64_t splits = (2 * (int64_t)sm_count() + all - 1) / all;
+  splits *= ((t.n + 4095) / 4096 + splits - 1) / splits;
   const int64_t most = (t.n + 63) / 64;
   splits = splits < most ? splits : most;
   bool vec = true;
