@@ -214,14 +214,17 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // turns, omega / pi folded in (products taken in double):
 //   w0u   [4][WP]     rows W0[:,0..2], b0 times omega0 / pi, then the largest
 //                     magnitude of each row
-//   ws_l  FP16 parts of W_l omega_l / pi 2^k_l (level_split.cuh), hi and lo; K
+//   ws_l  FP16 parts of W_l omega_l / pi 2^(k_l + d_n) (level_split.cuh), hi and lo; K
 //         blocks of kSplitK, block kb and part p at ((2 kb + p) WP kSplitK + ((n/8) (kSplitK/8) + (k%kSplitK)/8) 64
 //         + (n%8) 8 + k%8) elements
 //   us_l  [WP]        omega_l / pi b_l
 //   eq_l  [WP]        2^p_n: hidden activations that can never exceed 2^-p_n are
-//         carried 2^p_n times larger, the next layer's column 2^-p_n smaller
-//   ub    [layers][4] bound of |phase| over the layer's rows, largest |omega / pi
-//         W 2^-p|, whether some p_n of the layer is not 0, 2^-k_l
+//         carried 2^p_n times larger, the next layer's column 2^-p_n smaller;
+//         then [WP] 2^-d_n: rows far below the layer's largest are packed 2^d_n
+//         times larger than the others
+//   ub    [layers][4] bound of |phase| over the layer's rows (infinite where some
+//         d_n is not 0), largest |omega / pi W 2^-p|, whether some p_n of the
+//         layer is not 0, 2^-k_l
 constexpr int kSplitK = 32;
 struct PackLayout {
   int32_t L;    // nn.Linear layers

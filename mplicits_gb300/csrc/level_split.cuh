@@ -8,10 +8,10 @@
 //                hidden activations whose bound is below 1 are scaled up to it
 //                (PackLayout::eq) so that layers of small rows lose nothing;
 //   weights      w' = w omega / pi times a power of two that puts the layer's
-//                largest into FP16's top binade (PackLayout::ub); in a row n
-//                of largest magnitude 2^e_n, hi is a multiple of 2^(e_n - 11),
-//                lo = FP16 of the rest (error <= 2^(e_n - 24) for rows down to
-//                2^-16 of the largest, whose lo parts are normal numbers).
+//                largest into FP16's top binade (PackLayout::ub), and a row far
+//                below it into the same (PackLayout::eq); in a row n of largest
+//                magnitude 2^e_n, hi is a multiple of 2^(e_n - 11), lo = FP16 of
+//                the rest (error <= 2^(e_n - 24)).
 // hi*hi products are multiples of 2^(e_n - 21), so their sum over K is exact in
 // the FP32 accumulator up to 2^24 units (|sum| <= 2^(e_n + 3); larger sums lose
 // their last bit, as an FP32 chain does at every step).  hi*lo and lo*hi go to a second
@@ -412,10 +412,20 @@ __global__ void __launch_bounds__(kThreads, 1) level_split_kernel(const LevelArg
       __syncwarp();
       if (lane == 0) mbar_arrive(dempty);
       if (far) {
+        // rows at a scale of their own have 2^d_n (phase - bias) + bias
+        const float* own = reinterpret_cast<const float*>(pk + a.lay.eq[l]) + WP;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
-          for (int j = 0; j < kU / 2; ++j) u[c][j] = wrap2(u[c][j]);
+          for (int j = 0; j < kU; j += 2) {
+            const int at = c * 64 + h * kU + j;
+            const float2 d = *reinterpret_cast<const float2*>(own + at);
+            float x, y;
+            f2unpack(u[c][j / 2], x, y);
+            if (d.x != 1.f) x = fmaf(x - bias[at], d.x, bias[at]);
+            if (d.y != 1.f) y = fmaf(y - bias[at + 1], d.y, bias[at + 1]);
+            u[c][j / 2] = wrap2(f2pack(x, y));
+          }
       }
     };
     auto sine = [&](uint64_t v, float& s0, float& s1) {

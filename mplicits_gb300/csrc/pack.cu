@@ -58,7 +58,7 @@ int make_layout(const MplNet* net, PackLayout* lay) {
   for (int l = 1; l <= L - 2; ++l) {
     lay->ws[l] = take((int64_t)WP * WP * 4);
     lay->us[l] = take((int64_t)WP * 4);
-    lay->eq[l] = take((int64_t)WP * 4);
+    lay->eq[l] = take((int64_t)2 * WP * 4);
   }
   lay->total = o;
   return MPL_OK;
@@ -158,6 +158,11 @@ __global__ void pack_range(const PackArgs a) {
   if (k == 0) atomicMax(reinterpret_cast<unsigned int*>(h.ub + 1), __float_as_uint(m));
 }
 
+// Rows more powers of two than this below their layer's largest are packed at a
+// scale of their own: at the layer's, the lo parts of a row at 2^-17 of it leave
+// FP16's normal range (phase of such a row 3e-7 off at 2^-17, 6e-5 at 2^-25).
+constexpr int kSplitRange = 14;
+
 // One block of WP threads per row of a hidden layer (blockIdx.y - 1), and one
 // (blockIdx.y = 0, x = 0) for the first and output layers: the whole image in
 // one launch (a training step packs the level it has just updated).
@@ -213,14 +218,21 @@ __global__ void pack_level(const PackArgs a) {
     h.bh[n] = bb;
     h.hb[n] = v;
   }
-  // split parts: 2^k puts the layer's largest magnitude into [2^14, 2^15]; the
+  // split parts: 2^k puts the layer's largest magnitude into [2^14, 2^15], or the
+  // row's own where that is more than kSplitRange powers of two smaller; the
   // row's hi parts are multiples of 2^(e - 11), e its own largest exponent
   const double wu = split_weight(h, w, k);
   const float mx = block_max(fabsf((float)wu));
-  const int k2 = 15 - magnitude_exponent(h.ub[1]);
-  if (n == 0 && k == 0) h.ub[3] = (float)pow2(-k2);
+  const int el = magnitude_exponent(h.ub[1]), er = magnitude_exponent(mx);
+  const bool own = mx > 0.f && isfinite(mx) && er < el - kSplitRange;
+  const int k2 = 15 - (own ? er : el);
+  if (k == 0) {
+    h.eq[WP + n] = own ? (float)pow2(er - el) : 1.f;
+    if (own) h.ub[0] = INFINITY;
+    if (n == 0) h.ub[3] = (float)pow2(el - 15);
+  }
   const double wn = wu * pow2(k2);
-  const int eu = magnitude_exponent(mx) + k2 - 11;
+  const int eu = er + k2 - 11;
   const double hi = rint(wn * pow2(-eu)) * pow2(eu);
   const int kk = k % kSplitK;
   __half* dst = h.ws + (int64_t)(k / kSplitK) * 2 * WP * kSplitK +
