@@ -218,7 +218,7 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 //         blocks of kSplitK, block kb and part p at ((2 kb + p) WP kSplitK + ((n/8) (kSplitK/8) + (k%kSplitK)/8) 64
 //         + (n%8) 8 + k%8) elements
 //   us_l  [WP]        omega_l / pi b_l
-//   eq_l  [WP]        2^p_n: hidden activations that can never exceed 2^-p_n are
+//   eq_l  [WP]        2^p_n: hidden activations that are mostly below 2^-p_n are
 //         carried 2^p_n times larger, the next layer's column 2^-p_n smaller;
 //         then [WP] 2^-d_n: rows far below the layer's largest are packed 2^d_n
 //         times larger than the others

@@ -5,7 +5,7 @@
 // they split exactly where it matters:
 //   activations  s in [-1, 1]:  hi = s rounded to a multiple of 2^-10 (exact
 //                in FP16), lo = s - hi rounded to FP16 (error <= 2^-23);
-//                hidden activations whose bound is below 1 are scaled up to it
+//                hidden activations that are usually small are scaled up to 1
 //                (PackLayout::eq) so that layers of small rows lose nothing;
 //   weights      w' = w omega / pi times a power of two that puts the layer's
 //                largest into FP16's top binade (PackLayout::ub), and a row far
@@ -140,6 +140,17 @@ __device__ __forceinline__ void split2(float s0, float s1, uint32_t& hi, uint32_
   f2unpack(h, a, b);
   hi = bf16::Operand<__half>::pack(a, b);
   f2unpack(l, a, b);
+  lo = bf16::Operand<__half>::pack(a, b);
+}
+
+// the same of scaled sines, up to 2^5: beyond 2, hi is rounded to FP16's 11 bits
+__device__ __forceinline__ void split2_scaled(float s0, float s1, uint32_t& hi, uint32_t& lo) {
+  const uint64_t s = f2pack(s0, s1);
+  float a, b;
+  f2unpack(fadd2(fadd2(s, both(12288.f)), both(-12288.f)), a, b);
+  hi = bf16::Operand<__half>::pack(a, b);
+  const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  f2unpack(ffma2(f2pack(h.x, h.y), both(-1.f), s), a, b);
   lo = bf16::Operand<__half>::pack(a, b);
 }
 
@@ -465,10 +476,10 @@ __global__ void __launch_bounds__(kThreads, 1) level_split_kernel(const LevelArg
             sine(u[c][j], s0, s1);
             if (eq) {
               const float2 e = *reinterpret_cast<const float2*>(eq + c * 64 + h * kU + 2 * j);
-              s0 *= e.x;
-              s1 *= e.y;
+              split2_scaled(s0 * e.x, s1 * e.y, hi[j], lo[j]);
+            } else {
+              split2(s0, s1, hi[j], lo[j]);
             }
-            split2(s0, s1, hi[j], lo[j]);
           }
 #pragma unroll
           for (int g = 0; g < kU / 8; ++g)
