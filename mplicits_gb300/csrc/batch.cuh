@@ -489,6 +489,7 @@ __global__ void __launch_bounds__(bf16::Epi<U>::kThreads, 1) batch_kernel(const 
       float* const Sp = info.S;
       const int store_mode = info.store_mode;
       const float bout = info.bout;
+      fence_proxy_async_smem();  // the slot's reads before the copies that refill it
       __syncwarp();
       if (lane == 0) mbar_arrive(&cfree[slot]);
 
