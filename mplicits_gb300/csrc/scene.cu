@@ -1013,14 +1013,10 @@ __device__ Search search(const View& S, V3 q, V3 qt, V3 n, float delta, float de
       tw = sm.touch[w] < tw ? sm.touch[w] : tw;
       tau = fminf(tau, sm.tau[w]);
       if (warp == 0 && w > 0) {
-        // every key dropped here is at least the last one kept
-        const uint64_t more = sm.cand[w][lane];
-        const uint64_t a31 = __shfl_sync(0xffffffffu, r.list, 31);
-        const uint64_t x = merge32(r.list, more, lane);
-        const uint64_t last = __shfl_sync(0xffffffffu, x, 31);
-        const bool full = ~a31 != 0 || __any_sync(0xffffffffu, more > last);
-        if (~last != 0 && full) tau = fminf(tau, word_key(last));
-        r.list = x;
+        // a full list may have lost keys, each at least the last one kept
+        r.list = merge32(r.list, sm.cand[w][lane], lane);
+        const uint64_t last = __shfl_sync(0xffffffffu, r.list, 31);
+        if (~last != 0) tau = fminf(tau, word_key(last));
       }
     }
   }
