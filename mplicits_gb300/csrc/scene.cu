@@ -32,11 +32,11 @@
 // brute-force minimum's comparison bit for bit.  calc_deltas searches once per
 // certified stretch of a vertex's ray instead of once per step (see below).
 //
-// Three launches per iteration (decide, search by warps, search by blocks): the
-// stopping rule max(delta) < max_delta couples all vertices, so iteration i
-// reads the maximum left by iteration i - 1 (a float per iteration, reduced
-// with one atomic per block) and returns at once when it is reached, passing
-// the value on; no host round trip.
+// One launch per iteration for small meshes, three (decide, search by warps, search
+// by blocks) for others: the stopping rule max(delta) < max_delta couples all
+// vertices, so iteration i reads the maximum left by iteration i - 1 (a float per
+// iteration, reduced with one atomic per block) and returns at once when it is
+// reached, passing the value on; no host round trip.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -79,6 +79,15 @@ constexpr int kSearchBlocks = 3;
 // take every search (the others would leave warps idle)
 constexpr int kHeavyWarps = 4;
 constexpr uint32_t kFewSearches = 16384;
+// Vertices up to which a step is one launch (deltas_fused), and its blocks per SM.
+// Below, three dependent launches a step and a thread per vertex cost more than the
+// searches.  100 steps of a sphere-like mesh, a torus and two parallel sheets, by one
+// launch and by three: 482 / 384 / 512 vertices 0.78 / 0.74 / 0.74 and 1.70 / 1.38 /
+// 1.57 ms, 16,022 / 16,224 / 16,200 vertices 2.4 / 2.3 / 2.0 and 3.7 / 2.9 / 2.8;
+// 32,514 / 24,576 / 32,768 4.6 / 3.1 / 3.4 and 4.4 / 2.4 / 2.9.  (Six blocks per SM:
+// 4514 vertices 1.32 instead of 1.15 ms; ten spill, 1.26.)
+constexpr int64_t kFusedVertices = 16384;
+constexpr int kFusedBlocks = 8;
 // entries in a search's ball from which a block takes it instead of a warp
 constexpr uint32_t kHeavy = 4096;
 
@@ -635,8 +644,8 @@ struct Bisect {
   float* __restrict__ out;
   float4* __restrict__ state;  // step, clear, upper, flags (int bits)
   uint2* __restrict__ wit;     // touch and close entries (kNone: none)
-  float* __restrict__ key;     // [kList][M]
-  uint32_t* __restrict__ ent;  // [kList][M]
+  float* __restrict__ key;     // [kList][M], with one launch a step [M][kList]
+  uint32_t* __restrict__ ent;  // as key
   uint32_t* __restrict__ todo;  // [M] vertices of this step that need a search
   uint32_t* __restrict__ heavy;  // [M] of these, the ones for a whole block
 };
@@ -1124,6 +1133,84 @@ __global__ void __launch_bounds__(kThreads) deltas_step(View S, Bisect B, float*
   block_max(wmax, maxd + it + 1);
 }
 
+// One vertex's step by a search, by a warp (kWarps = 1, which lists a heavy one for
+// the blocks and gives it up) or a block.  kFused: its lists are laid out by vertex.
+template <int kWarps, bool kFused>
+__device__ __forceinline__ void search_vertex(const View& S, const Bisect& B, int64_t i,
+                                              SearchShared<kWarps>& sm, float& wmax,
+                                              StepCount* ct) {
+  constexpr bool kBlock = kWarps > 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool lead = kBlock ? threadIdx.x == 0 : lane == 0;  // writes the state
+  const float eps = B.eps;
+  float* o = B.out + i * (B.C + 1);
+  const float delta = o[B.C];
+  const V3 n = {o[3], o[4], o[5]};
+  const V3 q = ray_point(B, i, delta, n);
+  float4 st = B.state[i];
+  int flags = __float_as_int(st.w);
+  uint2 wit = B.wit[i];
+  bool shrink;
+  // the stretch to certify: half as far again as delta (at least eight
+  // steps; a far ball costs more entries than the searches it saves: to four
+  // times delta 45.3 ms on the sphere mesh, twice 38.2, half again 38.5, a
+  // quarter 41.0), no farther than a delta known to be close or the end of
+  // the loop
+  float delta_t = delta + ((flags & kShort) ? 4.f * fabsf(st.x)
+                                            : fmaxf(0.5f * delta, 8.f * fabsf(st.x)));
+  delta_t = fminf(delta_t, B.max_delta + 2.f * fabsf(st.x));
+  delta_t = fmaxf(fminf(delta_t, st.z), delta * 1.00001f);
+  const V3 qt = ray_point(B, i, delta_t, n);
+  if ((flags & kPlain) || !(delta > 0.f) || !finite3(qt)) {
+    shrink = shrink_step_warp(S, q, delta, eps, lane);
+  } else {
+    const bool touched = wit.x != kNone && __fsub_rn(entry_dist_call(S.tris, q, wit.x), delta) <= eps;
+    const Search r = search<kWarps>(S, q, qt, n, delta, delta_t, eps, touched, sm);
+    if (kWarps == 1 && r.heavy) {
+      if (lane == 0) B.heavy[atomicAdd(&ct->heavy, 1u)] = (uint32_t)i;
+      __syncwarp();
+      return;
+    }
+    shrink = r.shrink;
+    if (r.touch != kNone) wit.x = r.touch;
+    if (r.close != kNone) wit.y = r.close;
+    if (r.certified && (!kBlock || warp == 0)) {
+      // keep the kList nearest triangles (entries of one triangle carry the
+      // same word); the next one ends the certified stretch
+      const uint64_t prev = __shfl_up_sync(0xffffffffu, r.list, 1);
+      const bool own = word_key(r.list) < r.clear && !(lane > 0 && prev == r.list);
+      const unsigned om = __ballot_sync(0xffffffffu, own);
+      const int rank = __popc(om & ((1u << lane) - 1u));
+      if (own && rank < kList) {
+        const int64_t at = kFused ? i * kList + rank : (int64_t)rank * B.M + i;
+        B.key[at] = word_key(r.list);
+        B.ent[at] = (uint32_t)r.list;
+      }
+      float clear = r.clear;
+      const unsigned nm = __ballot_sync(0xffffffffu, own && rank == kList);
+      if (nm) clear = fminf(clear, word_key(__shfl_sync(0xffffffffu, r.list, __ffs(nm) - 1)));
+      st.y = clear;
+      flags = (flags & ~(kCountMask | kShort)) | min(__popc(om), kList);
+      if (clear < delta_t) flags |= kShort;
+    }
+  }
+  if (shrink) st.z = fminf(st.z, delta);
+  const float nd = advance(shrink, delta, st.x, flags);
+  st.w = __int_as_float(flags);
+  // every warp has read the vertex's state before it changes
+  if (kBlock)
+    __syncthreads();
+  else
+    __syncwarp();
+  if (lead) {
+    B.state[i] = st;
+    B.wit[i] = wit;
+    o[B.C] = nd;
+    wmax = fmaxf(wmax, nd);
+  }
+  __syncwarp();
+}
+
 // Second half: the listed vertices, one per warp (kWarps = 1) or one per block
 // of kWarps warps at a time, handed out by a counter: a search's cost varies by
 // a hundred between the mesh's sparse and dense parts, which lie together in
@@ -1148,8 +1235,6 @@ __global__ void __launch_bounds__(kWarps > 1 ? kWarps * 32 : kThreads,
   const bool few = ct.listed <= kFewSearches;
   const uint32_t total = kBlock ? (few ? ct.listed : ct.heavy) : (few ? 0u : ct.listed);
   const uint32_t* todo = kBlock && !few ? B.heavy : B.todo;
-  const bool lead = kBlock ? threadIdx.x == 0 : lane == 0;  // writes the state
-  const float eps = B.eps;
   float wmax = 0.f;
   for (;;) {
     uint32_t t = 0;
@@ -1163,72 +1248,81 @@ __global__ void __launch_bounds__(kWarps > 1 ? kWarps * 32 : kThreads,
       t = __shfl_sync(0xffffffffu, t, 0);
     }
     if (t >= total) break;
-    const int64_t i = todo[t];
-    float* o = B.out + i * (B.C + 1);
-    const float delta = o[B.C];
-    const V3 n = {o[3], o[4], o[5]};
-    const V3 q = ray_point(B, i, delta, n);
-    float4 st = B.state[i];
-    int flags = __float_as_int(st.w);
-    uint2 wit = B.wit[i];
-    bool shrink;
-    // the stretch to certify: half as far again as delta (at least eight
-    // steps; a far ball costs more entries than the searches it saves: to four
-    // times delta 45.3 ms on the sphere mesh, twice 38.2, half again 38.5, a
-    // quarter 41.0), no farther than a delta known to be close or the end of
-    // the loop
-    float delta_t = delta + ((flags & kShort) ? 4.f * fabsf(st.x)
-                                              : fmaxf(0.5f * delta, 8.f * fabsf(st.x)));
-    delta_t = fminf(delta_t, B.max_delta + 2.f * fabsf(st.x));
-    delta_t = fmaxf(fminf(delta_t, st.z), delta * 1.00001f);
-    const V3 qt = ray_point(B, i, delta_t, n);
-    if ((flags & kPlain) || !(delta > 0.f) || !finite3(qt)) {
-      shrink = shrink_step_warp(S, q, delta, eps, lane);
-    } else {
-      const bool touched = wit.x != kNone && __fsub_rn(entry_dist_call(S.tris, q, wit.x), delta) <= eps;
-      const Search r = search<kWarps>(S, q, qt, n, delta, delta_t, eps, touched, sm);
-      if (r.heavy) {
-        if (lane == 0) B.heavy[atomicAdd(&ct.heavy, 1u)] = (uint32_t)i;
-        __syncwarp();
-        continue;
-      }
-      shrink = r.shrink;
-      if (r.touch != kNone) wit.x = r.touch;
-      if (r.close != kNone) wit.y = r.close;
-      if (r.certified && (!kBlock || warp == 0)) {
-        // keep the kList nearest triangles (entries of one triangle carry the
-        // same word); the next one ends the certified stretch
-        const uint64_t prev = __shfl_up_sync(0xffffffffu, r.list, 1);
-        const bool own = word_key(r.list) < r.clear && !(lane > 0 && prev == r.list);
-        const unsigned om = __ballot_sync(0xffffffffu, own);
-        const int rank = __popc(om & ((1u << lane) - 1u));
-        if (own && rank < kList) {
-          B.key[(int64_t)rank * B.M + i] = word_key(r.list);
-          B.ent[(int64_t)rank * B.M + i] = (uint32_t)r.list;
-        }
-        float clear = r.clear;
-        const unsigned nm = __ballot_sync(0xffffffffu, own && rank == kList);
-        if (nm) clear = fminf(clear, word_key(__shfl_sync(0xffffffffu, r.list, __ffs(nm) - 1)));
-        st.y = clear;
-        flags = (flags & ~(kCountMask | kShort)) | min(__popc(om), kList);
-        if (clear < delta_t) flags |= kShort;
+    search_vertex<kWarps, false>(S, B, todo[t], sm, wmax, &ct);
+  }
+  block_max(wmax, maxd + it + 1);
+}
+
+// The same step by a warp: a lane per listed triangle, one for the touching one and
+// one for the last close one.  True: decided (and the state written).
+__device__ __forceinline__ bool decide_by_warp(const View& S, const Bisect& B, int64_t i, int lane,
+                                               float& wmax) {
+  float* o = B.out + i * (B.C + 1);
+  const float delta = o[B.C];
+  float4 st = B.state[i];
+  int flags = __float_as_int(st.w);
+  if (flags & kDone) {
+    wmax = fmaxf(wmax, delta);
+    return true;
+  }
+  const V3 q = ray_point(B, i, delta, {o[3], o[4], o[5]});
+  bool shrink = false;
+  if (finite3(q)) {
+    if (flags & kPlain) return false;
+    const uint2 wit = B.wit[i];
+    const bool inside = delta < st.y;  // of the certified stretch
+    uint32_t e = lane == 0 ? wit.x : (lane == 1 && !inside ? wit.y : kNone);
+    if (inside && lane >= 2 && lane - 2 < (flags & kCountMask)) {
+      const int64_t at = i * kList + lane - 2;
+      if (!(B.key[at] > delta)) e = B.ent[at];
+    }
+    const float d = e != kNone ? entry_dist(S, q, e) : 0.f;
+    const bool hit = e != kNone && (lane == 0 ? __fsub_rn(d, delta) <= B.eps
+                                              : __fsub_rn(delta, d) > B.eps);
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    shrink = m > 1u;
+    if (!(m & 1u) || (!inside && !shrink)) return false;
+    if (inside && shrink && lane == __ffs(m & ~1u) - 1) B.wit[i].y = e;
+  }
+  if (shrink) st.z = fminf(st.z, delta);
+  const float nd = advance(shrink, delta, st.x, flags);
+  st.w = __int_as_float(flags);
+  __syncwarp();  // every lane has read the state
+  if (lane == 0) {
+    B.state[i] = st;
+    o[B.C] = nd;
+  }
+  wmax = fmaxf(wmax, nd);
+  return true;
+}
+
+// A step in one launch, for meshes of up to kFusedVertices: a block of kHeavyWarps
+// warps takes `per` vertices at a time, a warp decides each from its lists, and the
+// block searches together for those that are left.
+__global__ void __launch_bounds__(kHeavyWarps * 32, kFusedBlocks)
+    deltas_fused(View S, Bisect B, float* maxd, int it, int per) {
+  const float before = maxd[it];
+  if (!(before < B.max_delta)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) maxd[it + 1] = before;
+    return;
+  }
+  __shared__ SearchShared<kHeavyWarps> sm;
+  __shared__ bool left[kHeavyWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float wmax = 0.f;
+  for (int64_t i0 = (int64_t)blockIdx.x * per; i0 < B.M; i0 += (int64_t)gridDim.x * per) {
+    const bool own = warp < per && i0 + warp < B.M;
+    const bool decided = !own || decide_by_warp(S, B, i0 + warp, lane, wmax);
+    if (lane == 0) left[warp] = !decided;
+    __syncthreads();
+#pragma unroll 1
+    for (int w = 0; w < per; ++w) {
+      if (left[w]) {
+        search_vertex<kHeavyWarps, true>(S, B, i0 + w, sm, wmax, nullptr);
+        __syncthreads();  // its shared memory is read
       }
     }
-    if (shrink) st.z = fminf(st.z, delta);
-    const float nd = advance(shrink, delta, st.x, flags);
-    st.w = __int_as_float(flags);
-    // every warp has read the vertex's state before it changes
-    if (kBlock)
-      __syncthreads();
-    else
-      __syncwarp();
-    if (lead) {
-      B.state[i] = st;
-      B.wit[i] = wit;
-      o[B.C] = nd;
-      wmax = fmaxf(wmax, nd);
-    }
-    __syncwarp();
+    __syncthreads();  // `left` is read
   }
   block_max(wmax, maxd + it + 1);
 }
@@ -1510,7 +1604,17 @@ extern "C" int mpl_calc_deltas(const MplScene* scene, const float* vertices_dev,
   const unsigned nsearch = (unsigned)(want < cap ? want : cap);
   const int64_t hcap = cap * 8 / kHeavyWarps;
   const unsigned nheavy = (unsigned)(n_vertices < hcap ? n_vertices : hcap);
+  const int64_t resident = (int64_t)sm_count() * kFusedBlocks;
+  const int64_t share = (n_vertices + resident - 1) / resident;
+  const int per = share < kHeavyWarps ? (int)share : kHeavyWarps;
+  const int64_t groups = (n_vertices + per - 1) / per;
+  const unsigned nfused = (unsigned)(groups < resident ? groups : resident);
   for (int it = 0; it < n_iters; ++it) {
+    if (n_vertices <= kFusedVertices) {
+      deltas_fused<<<nfused, kHeavyWarps * 32, 0, s>>>(v, B, maxd, it, per);
+      MPL_LAUNCH_CHECK();
+      continue;
+    }
     deltas_step<<<blocks(n_vertices), kThreads, 0, s>>>(v, B, maxd, count, it);
     MPL_LAUNCH_CHECK();
     deltas_search<1><<<nsearch, kThreads, 0, s>>>(v, B, maxd, count, it);
