@@ -73,12 +73,15 @@ constexpr int kScanBlock = kThreads * kScanItems;
 // calc_deltas: triangles a vertex keeps between iterations
 constexpr int kList = 16;
 // resident blocks per SM of its search kernels (four spill: 48.3 against 45.3 ms
-// on the sphere mesh)
+// on the 523,266-vertex sphere mesh; two 43.1 against 37.4, a torus of 240,000
+// vertices 10.9 against 9.3)
 constexpr int kSearchBlocks = 3;
-// warps that share a heavy search, and the listed vertices up to which they
-// take every search (the others would leave warps idle)
+// Warps that share a heavy search, and the listed vertices up to which they take
+// every search (the others would leave warps idle).  4096 / 8192 / 16384 / 32768
+// listed: sheets of 32,768 vertices 2.57 / 2.58 / 2.91 / 3.77 ms, the sphere mesh of
+// 32,514 4.37 / 4.37 / 4.38 / 5.54 and of 523,266 37.9 / 37.5 / 37.4 / 37.7.
 constexpr int kHeavyWarps = 4;
-constexpr uint32_t kFewSearches = 16384;
+constexpr uint32_t kFewSearches = 8192;
 // Vertices up to which a step is one launch (deltas_fused), and its blocks per SM.
 // Below, three dependent launches a step and a thread per vertex cost more than the
 // searches.  100 steps of a sphere-like mesh, a torus and two parallel sheets, by one
@@ -88,7 +91,8 @@ constexpr uint32_t kFewSearches = 16384;
 // 4514 vertices 1.32 instead of 1.15 ms; ten spill, 1.26.)
 constexpr int64_t kFusedVertices = 16384;
 constexpr int kFusedBlocks = 8;
-// entries in a search's ball from which a block takes it instead of a warp
+// entries in a search's ball from which a block takes it instead of a warp (2048 and
+// 8192: within 1% on the same meshes, but 38.0 and 37.8 ms on the largest)
 constexpr uint32_t kHeavy = 4096;
 
 struct View {
