@@ -1422,17 +1422,24 @@ extern "C" int mpl_scene_create(const float* positions_dev, int64_t n_positions,
   float ext = 0.f;
   for (int k = 0; k < 3; ++k) ext = fmaxf(ext, hi[k] - lo[k]);
   if (!(h > 0.f)) h = ext > 0.f ? ext : 1.f;
-  // bound the cell count: each dimension <= kMaxDim, the product <= kMaxCells
+  // bound the cell count: each dimension <= kMaxDim (an entry's home cell has 10 bits
+  // for each), the product <= kMaxCells.  1.25^1000 spans all of float's range.
   int64_t dim[3], cells = 0;
-  for (int guard = 0; guard < 64; ++guard) {
+  bool fits = false;
+  for (int guard = 0; guard < 1000 && !fits; ++guard) {
     cells = 1;
-    for (int k = 0; k < 3; ++k) {
-      dim[k] = (int64_t)((hi[k] - lo[k]) / h) + 3;
+    fits = true;
+    for (int k = 0; k < 3 && fits; ++k) {
+      const float n = (hi[k] - lo[k]) / h;
+      fits = n < (float)kMaxDim;  // false for an infinite extent too
+      dim[k] = fits ? (int64_t)n + 3 : 0;
+      fits = fits && dim[k] <= kMaxDim;
       cells *= dim[k];
     }
-    if (cells <= kMaxCells && dim[0] <= kMaxDim && dim[1] <= kMaxDim && dim[2] <= kMaxDim) break;
-    h *= 1.25f;
+    fits = fits && cells <= kMaxCells;
+    if (!fits) h *= 1.25f;
   }
+  if (!fits) return MPL_ERR_UNSUPPORTED;
 
   MplScene* sc = new MplScene();
   sc->device = dev;
