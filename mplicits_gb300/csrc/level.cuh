@@ -133,7 +133,9 @@ __device__ __forceinline__ void fp32_tile_thread(int tid, int& tx, int& ty) {
 // of its tiles can meet on one SM).  Gradient of n points, 256 wide, full and
 // half: 500 99.6 / 60.5 us, 4864 100 / 106, 6000 197 / 149, 7000 197 / 206,
 // 12,000 295 / 307, 30,000 683 / 657 (since then both forms are faster: half
-// tiles 500 54.6, 6000 129, 30,000 574 us; full ones 4864 88.7, 7000 175).
+// tiles 500 54.6, 6000 129, 30,000 574 us; full ones 4864 88.7, 7000 175).  At 128
+// wide the line lies in the same places: 500 63.5 / 53.9 us, 4865 89.1 / 77.2, 7000
+// 92.0 / 95.0, 11,000 120 / 104 (full ones taken), 14,592 123 / 125, 15,000 145 / 132.
 inline bool half_tiles(int64_t n, int WP) {
   if (WP < 128) return false;
   const int64_t sms = sm_count(), full = (n + 31) / 32, half = (n + 15) / 16;

@@ -2,7 +2,9 @@
 // over a point tile, FP32 SIMT FMAs, accurate sinf.  It serves the FP32
 // gradient and levels without a hidden GEMM; other FP32 levels run on the
 // tensor cores with split operands (level_split.cuh), ten times as fast and
-// with a smaller error.  One CTA per SM; a tile
+// with a smaller error.  The value beside a gradient is therefore not the
+// forward's bit for bit (other sums, both a few 1e-7 from float64).  One CTA per
+// SM; a tile
 // is 128 rows x the padded width WP; activations stay in shared memory
 // between layers; hidden-layer weights are streamed from L2 as 32-row
 // K-chunks by the TMA engine into a double buffer.  Replaces the per-layer
@@ -59,7 +61,7 @@ __global__ void __launch_bounds__(Fp32Threads<WP, kTile>::kThreads, kTile == 128
   float* wbuf = act + WP * kTile;                                // [2][KC][WP]
   float* w0t = wbuf + 2 * kKC * WP;                              // [3][WP]
   float* b0 = w0t + 3 * WP;                                      // [WP]
-  const int nh = a.lay.nh;
+  const int nh = GRAD ? a.lay.nh : 0;  // values of deeper levels: level_split.cuh
   float* bh = b0 + WP;                                           // [nh][WP]
   float* wout = bh + (nh > 0 ? nh : 1) * WP;                     // [WP]
   float* pts = wout + WP;                                        // [kTile][3]
@@ -371,10 +373,7 @@ int launch_fp32_mode(const LevelArgs& a, cudaStream_t s) {
 }  // namespace
 
 int launch_level_fp32(const LevelArgs& a, cudaStream_t s) {
-  if (!a.grad && a.lay.nh >= 1) {
-    const int st = launch_level_split(a, s);
-    if (st != MPL_ERR_UNSUPPORTED) return st;
-  }
+  if (!a.grad && a.lay.nh >= 1) return launch_level_split(a, s);
   return a.grad ? launch_fp32_mode<true>(a, s) : launch_fp32_mode<false>(a, s);
 }
 
