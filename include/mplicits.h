@@ -392,7 +392,8 @@ int mpl_scene_compute_distance(const MplScene* scene, const float* points_dev, i
  * in double for a Python float max_delta, in float32 for a float32 tensor,
  * then rounded to float32); the loop runs while max(delta) < max_delta,
  * n_iters times at most (the reference uses eps 2e-4).  scratch
- * is sized by mpl_calc_deltas_scratch_bytes (256-byte aligned).
+ * is sized by mpl_calc_deltas_scratch_bytes (256-byte aligned): about 160
+ * bytes a vertex for the certified stretches and lists, 84 MB for 523,266.
  * iterations_dev (nullable, device int32) receives the number of
  * iterations run.  Results equal the reference loop over an exact
  * nearest-triangle distance bit for bit. */

@@ -19,7 +19,12 @@ from . import capi
 def level_gradient(model, x, S=None, G=None, accumulate=False, precision=None, index=None,
                    n_dev=None, n=None):
     """(S, G): f(x) [P] and df/dx [P, 3] of one level.  With ``index`` the
-    points are x[index[q]] and the results land at S[index[q]], G[index[q]]."""
+    points are x[index[q]] and the results land at S[index[q]], G[index[q]].
+
+    In "fp32" the value comes from the FMA kernel, that of ``SIREN.forward``
+    from the split-operand kernel: both a few 1e-7 (2-norm) from float64, with
+    sums in another order, so a value next to a threshold can fall on either
+    side."""
     if not x.is_cuda:
         raise RuntimeError("mplicits_gb300 evaluates levels on a CUDA device only")
     x = x.detach().float().contiguous()

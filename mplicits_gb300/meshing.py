@@ -100,7 +100,7 @@ class BandedReconstruction:
     a band threshold are re-evaluated with the FP32 kernels before the band
     list is cut, and points with |S| < m after the last level get every level
     in FP32, so the band decisions and the marching-cubes signs are those of
-    the plain FP32 path.
+    the FP32 path.
 
     Band widths that never grow from one level to the next (the usual case)
     make each band a subset of the previous one, so every level cuts the next

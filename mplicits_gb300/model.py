@@ -175,8 +175,9 @@ def level_forward(model, x, S=None, accumulate=False, precision=None):
 class SIREN(nn.Module):
     """SIREN level with the signature of i3d.model.SIREN (i3d/model.py:76-105).
 
-    Extra attribute ``precision`` ("fp32" plain form, default; or "bf16" for
-    the tcgen05 hidden GEMMs) selects the kernel of ``forward``.
+    Extra attribute ``precision`` selects the kernel of ``forward``: "fp32"
+    (default; FP32 accuracy, split operands on the tensor cores), "bf16" or
+    "fp16" (hidden GEMMs on operands of 16 bits).
     """
 
     def __init__(self, n_in_features, n_out_features, hidden_layer_config=[], w0=30, ww=None,

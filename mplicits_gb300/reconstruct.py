@@ -4,7 +4,7 @@
 Same positional arguments and flags, same printed lines and the same
 ``SAMPLING_TIME_S:<seconds>`` line that reproduce.py parses; the band-culled
 evaluation and marching cubes run on the GPU through libmplicits.  New flag:
-``--precision {fp32,bf16,fp16}`` (fp32, the plain form, is the default).
+``--precision {fp32,bf16,fp16}`` (fp32 is the default).
 ``--input`` reads the training point cloud from a PLY file (ASCII or binary
 vertex x/y/z), which the reference reads with open3d.
 """
@@ -124,7 +124,7 @@ def main(argv=None):
     parser.add_argument("--deltas", type=float, nargs="+", default=None,
                         help="Explicit band widths (one per residual level).")
     parser.add_argument("--precision", choices=["fp32", "bf16", "fp16"], default="fp32",
-                        help="Arithmetic of the hidden layers: fp32 (plain form), or bf16 / "
+                        help="Arithmetic of the hidden layers: fp32 accuracy, or bf16 / "
                              "fp16 operands on the tcgen05 tensor cores.")
     args = parser.parse_args(argv)
     out_dir = osp.split(args.output_path)[0]
