@@ -256,6 +256,7 @@ class ResidualTrainer:
         self.exp_avg_sq = [torch.zeros_like(p) for p in self.params]
         self.t = 0
         self.loss_sums = torch.zeros(4, dtype=torch.float32, device=self.params[0].device)
+        self._scale_n = None  # (n, scale / n) of the last batch size
         self._scale = torch.tensor([w[k] for k in self.names], dtype=torch.float32,
                                    device=self.params[0].device)
 
@@ -266,9 +267,16 @@ class ResidualTrainer:
         return self._loss_and_grads(x, normals, sdf, own=True)
 
     def _terms(self, n):
-        """The weighted loss terms from the sums over n points (scale / n is not
-        kept: made while a CUDA graph is captured, it has no value outside it)."""
-        return self.loss_sums[:len(self.names)] * (self._scale / n)
+        """The weighted loss terms from the sums over n points.  scale / n is kept
+        for the last batch size, but a CUDA graph makes its own: one made while a
+        graph is captured has no value outside it, and the kept one goes when
+        another batch size comes."""
+        kept = self._scale_n
+        if torch.cuda.is_current_stream_capturing():
+            kept = (n, self._scale / n)
+        elif kept is None or kept[0] != n:
+            kept = self._scale_n = (n, self._scale / n)
+        return self.loss_sums[:len(self.names)] * kept[1]
 
     def _loss_and_grads(self, x, normals, sdf, own):
         x = x.detach().float().reshape(-1, 3).contiguous()

@@ -35,3 +35,25 @@ def test_eager_after_capture(precision):
     graph.replay()
     torch.cuda.synchronize()
     assert (captured - want).abs().max() <= tol
+
+
+def test_replay_after_other_batch_sizes():
+    from mplicits_gb300.model import SIREN
+    from mplicits_gb300.train import ResidualTrainer
+    torch.manual_seed(0)
+    m = SIREN(3, 1, [128, 128, 128], w0=30).cuda()
+    tr = ResidualTrainer(m)
+    tr.loss_and_grads(*_batch(500, 2))
+    batch = _batch(300, 1)
+    want = tr.loss_and_grads(*batch)[0].clone()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        captured, _ = tr.loss_and_grads(*batch)
+    for n in (400, 200, 100):
+        tr.loss_and_grads(*_batch(n, 3))
+        torch.full((3,), 1e30, device="cuda")  # takes up what was given back
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (captured - want).abs().max() <= 2e-5 * want.abs().max()
