@@ -202,7 +202,11 @@ class SIREN(nn.Module):
     def linears(self):
         # the first child of each block, whatever it is called (plain lookups:
         # indexing a Sequential costs a microsecond each)
-        return [next(iter(blk._modules.values())) for blk in self._modules["net"]._modules.values()]
+        blocks = self._modules["net"]._modules.values()
+        try:
+            return [blk._modules["0"] for blk in blocks]
+        except KeyError:
+            return [next(iter(blk._modules.values())) for blk in blocks]
 
     def omegas(self):
         out = []
